@@ -25,54 +25,48 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   return v;
 }
 
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // ------------------------------------------------------------------ grid barrier
-// Generation barrier over all blocks of a co-resident (cooperative) grid. sync[0] counts
-// arrivals, sync[1] is the generation. Every wait is bounded: after kSpinLimit polls the block
-// records FLYB_EBARRIER in status and returns false; callers then return, so a grid that is not
-// co-resident ends with an error status instead of hanging.
+// Barrier over all blocks of a co-resident (cooperative) grid: sync[0], zero at the launch, counts
+// the arrivals of all barriers so far; barrier g is complete at (g + 1) x blocks arrivals. One
+// release add and one acquire load carry the ordering (the threads of a block are ordered by the
+// block barriers around them), about 1 us where separate fences, a return of the count and a
+// second generation word took 2-3. Every wait is bounded: after kSpinLimit polls the block records
+// FLYB_EBARRIER in status and returns false; callers then return, so a grid that is not co-resident
+// ends with an error status instead of hanging.
 constexpr long long kSpinLimit = 1ll << 24;   // polls with a 64-256 ns backoff: seconds at most
 
-// Polls *p until it differs from `value`, at most `limit` times (or until status is set).
-// Returns false, with FLYB_EBARRIER recorded at `where`, when the limit ran out.
-__device__ __forceinline__ bool bounded_wait_ne(const int* p, int value, int* status, long long limit, int where,
-                                                int step) {
-  long long it = 0;
-  unsigned ns = 64;
-  while (ld_acquire(p) == value) {
-    if (++it > limit || ld_acquire(status) != 0) {
+// Polls *p until `done(value)` holds, at most `limit` times (or until status is set). Returns false,
+// with FLYB_EBARRIER recorded at `where`, when the limit ran out.
+template <typename Done>
+__device__ __forceinline__ bool bounded_wait(const int* p, Done done, int* status, long long limit, int where, int step) {
+  unsigned ns = 0;                              // the first polls follow each other: a short wait ends at once
+  for (long long it = 0; !done(ld_acquire(p)); ++it) {
+    if (it >= limit || ((it & 15) == 15 && ld_acquire(status) != 0)) {
       set_error(status, FLYB_EBARRIER, where, step);
       return false;
     }
+    if (it < 32) continue;
+    ns = ns < 64 ? 64 : (ns < 256 ? ns << 1 : ns);
     __nanosleep(ns);
-    if (ns < 256) ns <<= 1;
   }
   return true;
 }
 
+__device__ __forceinline__ bool bounded_wait_ne(const int* p, int value, int* status, long long limit, int where,
+                                                int step) {
+  return bounded_wait(p, [=](int v) { return v != value; }, status, limit, where, step);
+}
+
 __device__ __forceinline__ bool grid_barrier(int* sync, int* status, int& generation, int step) {
-  __syncthreads();
   __shared__ int ok;
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const int gen = generation;
-    __threadfence();
-    const int nblocks = gridDim.x * gridDim.y * gridDim.z;
-    const int arrived = atomicAdd(&sync[0], 1);
-    if (arrived == nblocks - 1) {
-      sync[0] = 0;
-      __threadfence();
-      st_release(&sync[1], gen + 1);
-    } else if (!bounded_wait_ne(&sync[1], gen, status, kSpinLimit, 1, step)) {
-      ok = 0;
-    }
-    __threadfence();
-  }
   __syncthreads();
   generation += 1;
+  if (threadIdx.x == 0) {
+    const unsigned target = (unsigned)generation * (gridDim.x * gridDim.y * gridDim.z);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync) : "memory");
+    ok = bounded_wait(sync, [=](int v) { return (int)((unsigned)v - target) >= 0; }, status, kSpinLimit, 1, step);
+  }
+  __syncthreads();
   return ok != 0;
 }
 

@@ -1467,6 +1467,12 @@ static int run_lif_ipt(const LifK& k, int launch, int grid_cap, cudaStream_t st)
   return (int)e;
 }
 
+}  // namespace flyb
+
+#include "lif_window.cuh"
+
+namespace flyb {
+
 // `ipt` items per thread (8- or 16-byte state vectors) need every ring slot and state array
 // aligned at each thread's first item: n * batch % ipt == 0 and (4 * ipt)-byte aligned bases.
 static bool vectorizable(const LifK& k, int ipt) {
@@ -1484,6 +1490,11 @@ template <int BLOCK, bool FIXED>
 static int run_lif(const LifK& k, int want, int launch, int grid_cap, int staged, cudaStream_t st) {
   int ipt = want ? want : 4;
   if (ipt != 1 && ipt != 2 && ipt != 4) return FLYB_EINVAL;
+  if (const int K = window_steps(k)) {
+    if constexpr (FIXED)        // depression runs on the fixed ring only
+      if (k.flags & FLYB_LIF_STD) return run_by_windows<FIXED, true>(k, K, launch, grid_cap, st);
+    return run_by_windows<FIXED, false>(k, K, launch, grid_cap, st);
+  }
   if (staged && launch == FLYB_LAUNCH_STEP && stageable(k))
     return ipt == 4 ? run_lif_staged<BLOCK, FIXED, 4>(k, grid_cap, st) : run_lif_staged<BLOCK, FIXED, 2>(k, grid_cap, st);
   while (ipt > 1 && !vectorizable(k, ipt)) ipt >>= 1;

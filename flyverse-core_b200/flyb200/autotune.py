@@ -62,13 +62,38 @@ def _time(fn, reps: int) -> float:
     return s.elapsed_time(e) / reps
 
 
+def _one_by_one(brain, steps: int) -> None:
+    """`steps` steps by single-step launches, as WholeFly takes them: the update over all neurons, the
+    clock, and under pull delivery a pull per complete group."""
+    for _ in range(steps):
+        brain.step_range(0, brain.n)
+        brain.advance(1, pull=False)
+        if brain._pull_active() and brain.step_count % brain.pull_group == 0:
+            brain.deliver()
+    brain.deliver()
+
+
+def _time_one_by_one(brain, steps: int) -> float:
+    """Milliseconds of `_one_by_one`, replayed from a CUDA graph: the host's time per launch is not
+    what the candidates differ in."""
+    stream, graph = torch.cuda.Stream(brain.device), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream(brain.device))
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        _one_by_one(brain, steps)
+    torch.cuda.current_stream(brain.device).wait_stream(stream)
+    graph.replay()
+    return _time(graph.replay, 1)
+
+
 def tune_lif(brain, steps: int = 10, candidates=LIF_CANDIDATES) -> dict:
     """Install and return the fastest LIF launch choice for this brain; state is left unchanged.
     A brain with per-neuron clocks or the slow receptor tone has one launch shape (the extended
-    kernel): nothing to tune."""
+    kernel): nothing to tune. Calls of several steps run by delay windows, whose update has one
+    shape too: there the candidates differ in the launch mode and the delivery. A brain that
+    is stepped one step per launch (`single_steps`, set by WholeFly) is timed that way."""
     if getattr(brain, "_kvec", None) is not None or getattr(brain, "slow", None) is not None:
         return {"launch": "step", "block": 256, "items_per_thread": 1, "delivery": "extended", "ms_per_step": None}
-    key = ("lif", graph_key(brain), brain.B, activity_bucket(brain))
+    key = ("lif", graph_key(brain), brain.B, activity_bucket(brain), bool(getattr(brain, "single_steps", False)))
     if key in CACHE:
         _apply(brain, CACHE[key])
         return CACHE[key]
@@ -78,8 +103,13 @@ def tune_lif(brain, steps: int = 10, candidates=LIF_CANDIDATES) -> dict:
         candidates = [c for c in candidates if "pull" not in c[3]]
     for launch, block, ipt, delivery in candidates:
         _apply(brain, {"launch": launch, "block": block, "items_per_thread": ipt, "delivery": delivery})
-        brain.step(2)
-        results[(launch, block, ipt, delivery)] = _time(lambda: brain.step(steps), 1) / steps
+        if getattr(brain, "single_steps", False):
+            _one_by_one(brain, 2)
+            ms = _time_one_by_one(brain, steps)
+        else:
+            brain.step(2)
+            ms = _time(lambda: brain.step(steps), 1)
+        results[(launch, block, ipt, delivery)] = ms / steps
         brain.load_state_dict(saved)
     best = min(results, key=results.get)
     choice = {"launch": best[0], "block": best[1], "items_per_thread": best[2], "delivery": best[3],

@@ -55,6 +55,7 @@ class WholeFly:
         self.lif = Brain(self.lif_connectome, LIFParams(**params), device=self.device, seed=seed, batch=self.B,
                          launch=launch)
         self.lif.record_activity = record_activity
+        self.lif.single_steps = True                      # the tuner times what step() launches
         hz = cfg.lif.poisson_hz if poisson_hz is None else poisson_hz
         self.lif.set_poisson(self.sensory_idx, torch.as_tensor(hz, dtype=torch.float32))
         self.overlap = bool(overlap)

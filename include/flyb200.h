@@ -92,8 +92,12 @@ int launch_means(void** p, int n, int groups, int batch, int stride, void* strea
 #define FLYB_RING_FIXED  1   /* int64 Q32.32 millivolts; each edge rounds w*x once (exact sum)  */
 
 /* Launch modes */
-#define FLYB_LAUNCH_STEP       0   /* one kernel launch per step (the "plain" kernel)        */
-#define FLYB_LAUNCH_PERSISTENT 1   /* one cooperative launch for all steps, grid barrier/step */
+#define FLYB_LAUNCH_STEP       0   /* kernel launches per step (the "plain" kernel)           */
+#define FLYB_LAUNCH_PERSISTENT 1   /* one cooperative launch for all steps                    */
+/* An LIF run of nsteps >= 2 with a raster, n_delay >= 2 and no episode counters goes by delay
+ * windows under both launch modes: up to min(n_delay, raster_slots, 32) steps per pass over the
+ * state, then the delivery of their spikes (a pull: windows of at most two groups). block,
+ * items_per_thread, staged and FLYB_LIF_DEFER_DELIVERY shape single-step launches only.        */
 
 #define FLYB_SLOW_MAX_CLASSES 2   /* slow receptor classes: classical metabotropic, monoamine */
 
