@@ -3,8 +3,8 @@
 // (optic.py:579-580, 599-602) and the reference-compatible elementwise / CSR launchers.
 //
 // Layout: state [m][batch] (unit-major, fly-minor); CSR entries interleaved as int2 {col, w bits}.
-// A warp holds 32/LPR row slots; in a slot F lanes span the flies (FPL consecutive flies each: a
-// 4-, 8- or 16-byte vector gather of x[col][*]) and LPR/F lane groups split the entries, each lane
+// A warp holds 32/LPR row slots; in a slot F lanes span the flies (NV vectors of W consecutive flies
+// each: 4-, 8- or 16-byte gathers of x[col][*]) and LPR/F lane groups split the entries, each lane
 // keeping U independent gathers in flight. Rows run longest first; rows longer than a threshold
 // are split over every slot of a block and summed through shared memory. The gathered vector
 // (dr, 0.36 MB per fly) stays L2-resident; the CSR streams from HBM once per substep for all flies.
@@ -31,11 +31,6 @@ struct OpticK {
   int dr_valid;                   // buf0 already holds clip(v + b) - b: no initialisation pass
 };
 
-template <int FPL> struct VecT;
-template <> struct VecT<1> { using T = float; };
-template <> struct VecT<2> { using T = float2; };
-template <> struct VecT<4> { using T = float4; };
-
 template <int FPL>
 __device__ __forceinline__ void load_x(const float* __restrict__ p, float (&x)[FPL]) {
   if constexpr (FPL == 1) {
@@ -58,51 +53,86 @@ __device__ __forceinline__ void load_x(const float* __restrict__ p, float (&x)[F
 template <int FPL>
 struct Unroll { static constexpr int U = FPL <= 2 ? 8 : (FPL == 4 ? 4 : 2); };
 
-// acc[q] = sum over the row of w * x[col][f*FPL + q] for this lane's flies, for the row of this
-// lane's slot: a warp holds 32/LPR row slots of LPR lanes; within a slot, F lanes span the flies
-// (FPL consecutive flies each) and G = LPR/F lane groups split the entries (group g takes entries
-// e0 + g + G*k). Each pass loads U interleaved {col, w} entries (8 bytes each), issues U
-// independent gathers, then accumulates them with FMAs. The result is complete on the lanes with
-// slot lane < F. `row_ok` false: the lane still takes part in the shuffles.
-template <int F, int FPL, int LPR, int U = Unroll<FPL>::U>
-__device__ __forceinline__ void row_product(const int* __restrict__ ptr, const int2* __restrict__ cw,
-                                            const float* __restrict__ x, int batch, int row, bool row_ok,
-                                            float (&acc)[FPL], int part = 0, int parts = 1) {
+// How the flies of a unit lie on the F fly lanes of a row slot: W consecutive flies per vector (a 4-,
+// 8- or 16-byte access, W dividing the batch), NV vectors per lane, F vectors apart. A lane's
+// vector is inside the batch as a whole or not at all.
+template <int W, int NV, int F>
+struct Flies {
+  static constexpr int FPL = W * NV;                               // flies per lane
+  static __device__ __forceinline__ int at(int f, int v) { return (f + v * F) * W; }
+};
+
+template <int W>
+__device__ __forceinline__ void load_w(const float* p, float* x) {
+  if constexpr (W == 1) {
+    x[0] = *p;
+  } else if constexpr (W == 2) {
+    const float2 q = *reinterpret_cast<const float2*>(p); x[0] = q.x; x[1] = q.y;
+  } else {
+    const float4 q = *reinterpret_cast<const float4*>(p); x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void store_w(float* p, const float* x) {
+  if constexpr (W == 1) *p = x[0];
+  else if constexpr (W == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  else *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+
+// One {column, weight} entry. Where one load of the warp covers whole sectors of entries (4 lane
+// groups or more) the entries leave L1 to the gathered vector, much of which stays there at one
+// fly (0.36 MB against 0.2 MB of L1); with fewer groups the next loads of the warp read the
+// rest of the same sector from L1 (128 flies: 416 us a substep, 526 us without).
+template <bool STREAM>
+__device__ __forceinline__ int2 load_entry(const int2* p) {
+  if constexpr (!STREAM) return __ldg(p);
+  int2 c;
+  asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(c.x), "=r"(c.y) : "l"(p));
+  return c;
+}
+
+// acc = sum over the row of w * x[col][flies of this lane], for the row of this lane's slot: a warp
+// holds 32/LPR row slots of LPR lanes; within a slot, F lanes span the flies and G = LPR/F lane
+// groups split the entries (group g takes entries e0 + g + G*k). Each pass loads U entries per
+// lane, issues U independent gathers, then accumulates them with FMAs. The result is complete on
+// the lanes with slot lane < F. An empty row still takes part in the shuffles. A lane without flies
+// gathers fly 0: no predicate stands around the gathers.
+template <int W, int NV, int F, int LPR, int U>
+__device__ __forceinline__ void row_product(const int2* __restrict__ cw, const float* x, int batch, int e0, int e1,
+                                            float (&acc)[W * NV], int part = 0, int parts = 1) {
   static_assert(F <= LPR && LPR <= 32, "a row slot spans the fly lanes");
-  constexpr int G = LPR / F;
+  constexpr int G = LPR / F, FPL = W * NV;
   const int sl = (threadIdx.x & 31) % LPR, g = sl / F, f = sl % F;
-  const int fb = f * FPL;
-  const bool full = batch == F * FPL;
+  const float* xl[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int fly = Flies<W, NV, F>::at(f, v);
+    xl[v] = x + (fly < batch ? fly : 0);
+  }
   const int stride = parts * G;          // `parts` slots share a long row: slot `part` takes every parts-th group
 #pragma unroll
   for (int q = 0; q < FPL; ++q) acc[q] = 0.0f;
-  if (row_ok) {
-    const int e0 = __ldg(&ptr[row]), e1 = __ldg(&ptr[row + 1]);
-    for (int base = e0 + part * G + g; base < e1; base += stride * U) {
-      int2 c[U];
+  for (int base = e0 + part * G + g; base < e1; base += stride * U) {
+    int2 c[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int e = base + u * stride;
-        c[u] = e < e1 ? __ldg(&cw[e]) : make_int2(-1, 0);
-      }
-      float xv[U][FPL];
+    for (int u = 0; u < U; ++u) {
+      const int e = base + u * stride;
+      c[u] = e < e1 ? load_entry<(G >= 4)>(&cw[e]) : make_int2(-1, 0);
+    }
+    float xv[U][FPL];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float* xp = x + ((c[u].x < 0 ? 0 : c[u].x) * batch + fb);
-        if (full) {
-          load_x<FPL>(xp, xv[u]);
-        } else {
+    for (int u = 0; u < U; ++u) {
+      const int off = (c[u].x < 0 ? 0 : c[u].x) * batch;
 #pragma unroll
-          for (int q = 0; q < FPL; ++q) xv[u][q] = fb + q < batch ? __ldg(xp + q) : 0.0f;
-        }
-      }
+      for (int v = 0; v < NV; ++v) load_w<W>(xl[v] + off, &xv[u][v * W]);
+    }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (c[u].x >= 0) {
-          const float wv = __int_as_float(c[u].y);
+    for (int u = 0; u < U; ++u) {
+      if (c[u].x >= 0) {
+        const float wv = __int_as_float(c[u].y);
 #pragma unroll
-          for (int q = 0; q < FPL; ++q) acc[q] = fmaf(wv, xv[u][q], acc[q]);
-        }
+        for (int q = 0; q < FPL; ++q) acc[q] = fmaf(wv, xv[u][q], acc[q]);
       }
     }
   }
@@ -112,105 +142,88 @@ __device__ __forceinline__ void row_product(const int* __restrict__ ptr, const i
     for (int q = 0; q < FPL; ++q) acc[q] = acc[q] + __shfl_xor_sync(0xffffffffu, acc[q], o);
 }
 
-// The fused rate update of one (unit, fly), reference order (neural.cu:68-79, optic.py:528-551).
-__device__ __forceinline__ void optic_update(const OpticK& k, int s, size_t t, int i, float y,
-                                             const float* __restrict__ dr_in, float* __restrict__ dr_out) {
-  const float old = dr_in[t];
-  float inp = k.gr * y;
-  inp = inp + k.pr[t];
-  const float ad = k.ga * k.adapt[t];
-  inp = inp - ad;
-  inp = inp + k.spk[t];
-  float vv = k.v[t];
-  const size_t sz = (size_t)k.m * k.batch;
-  if (k.v_hist) k.v_hist[(size_t)s * sz + t] = vv;
-  if (k.inp_hist) k.inp_hist[(size_t)s * sz + t] = inp;
-  float dv = vv - inp;
-  dv = dv * k.a[i];
-  vv = inp + dv;
-  k.v[t] = vv;
-  float da = k.adapt[t] - old;
-  da = da * k.aad;
-  k.adapt[t] = old + da;
-  const float bb = k.b[i];
-  const float r = clip01(vv + bb);
-  dr_out[t] = r - bb;
+// What the update of one unit reads, for W flies.
+template <int W>
+struct UnitIn { float old[W], pr[W], spk[W], ad[W], vv[W]; };
+
+template <int W>
+__device__ __forceinline__ void load_unit(const OpticK& k, size_t t, const float* dr_in, UnitIn<W>& x) {
+  load_w<W>(dr_in + t, x.old);
+  load_w<W>(k.pr + t, x.pr);
+  load_w<W>(k.spk + t, x.spk);
+  load_w<W>(k.adapt + t, x.ad);
+  load_w<W>(k.v + t, x.vv);
 }
 
-template <int FPL>
-__device__ __forceinline__ void store_x(float* p, const float (&x)[FPL]) {
-  if constexpr (FPL == 1) {
-    *p = x[0];
-  } else if constexpr (FPL == 2) {
-    *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-  } else {
-#pragma unroll
-    for (int q = 0; q < FPL; q += 4) *reinterpret_cast<float4*>(p + q) = make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
-  }
-}
-
-// The same update for FPL consecutive flies of one unit with vector loads and stores (batch == F*FPL).
-template <int FPL>
-__device__ __forceinline__ void optic_update_vec(const OpticK& k, int s, size_t t, int i, const float (&y)[FPL],
-                                                 const float* __restrict__ dr_in, float* __restrict__ dr_out) {
-  float old[FPL], pr[FPL], spk[FPL], ad[FPL], vv[FPL];
-  load_x<FPL>(dr_in + t, old);
-  load_x<FPL>(k.pr + t, pr);
-  load_x<FPL>(k.spk + t, spk);
-  load_x<FPL>(k.adapt + t, ad);
-  load_x<FPL>(k.v + t, vv);
+// The fused rate update of W flies of unit i, reference order (neural.cu:68-79, optic.py:528-551).
+template <int W>
+__device__ __forceinline__ void update_unit(const OpticK& k, int s, size_t t, int i, const float* y, const UnitIn<W>& x,
+                                            float* dr_out) {
   const float ai = k.a[i], bb = k.b[i];
   const size_t sz = (size_t)k.m * k.batch;
-  if (k.v_hist) store_x<FPL>(k.v_hist + (size_t)s * sz + t, vv);
-  float inpv[FPL], nv[FPL], na[FPL], nd[FPL];
+  if (k.v_hist) store_w<W>(k.v_hist + (size_t)s * sz + t, x.vv);
+  float inpv[W], nv[W], na[W], nd[W];
 #pragma unroll
-  for (int q = 0; q < FPL; ++q) {
+  for (int q = 0; q < W; ++q) {
     float inp = k.gr * y[q];
-    inp = inp + pr[q];
-    const float a2 = k.ga * ad[q];
+    inp = inp + x.pr[q];
+    const float a2 = k.ga * x.ad[q];
     inp = inp - a2;
-    inp = inp + spk[q];
+    inp = inp + x.spk[q];
     inpv[q] = inp;
-    float dv = vv[q] - inp;
+    float dv = x.vv[q] - inp;
     dv = dv * ai;
     nv[q] = inp + dv;
-    float da = ad[q] - old[q];
+    float da = x.ad[q] - x.old[q];
     da = da * k.aad;
-    na[q] = old[q] + da;
+    na[q] = x.old[q] + da;
     nd[q] = clip01(nv[q] + bb) - bb;
   }
-  if (k.inp_hist) store_x<FPL>(k.inp_hist + (size_t)s * sz + t, inpv);
-  store_x<FPL>(k.v + t, nv);
-  store_x<FPL>(k.adapt + t, na);
-  store_x<FPL>(dr_out + t, nd);
+  if (k.inp_hist) store_w<W>(k.inp_hist + (size_t)s * sz + t, inpv);
+  store_w<W>(k.v + t, nv);
+  store_w<W>(k.adapt + t, na);
+  store_w<W>(dr_out + t, nd);
 }
 
-// y (FPL flies of slot lane sl) -> the fused update of one unit.
-template <int F, int FPL>
-__device__ __forceinline__ void optic_epilogue(const OpticK& k, int s, int row, int sl, const float (&y)[FPL],
-                                               const float* dr_in, float* dr_out) {
-  if (k.batch == F * FPL) {
-    optic_update_vec<FPL>(k, s, (size_t)row * k.batch + sl * FPL, row, y, dr_in, dr_out);
-  } else {
+// The product of a row (`product` fills y) and the update of its unit on the slot's fly lanes. With
+// one or two flies per lane the update's operands are requested before the product: their latency
+// then passes beside the row's gathers instead of after them (with four the registers cost more
+// warps than that gains: 64 us against 38 at four flies).
+template <int W, int NV, int F, typename Product>
+__device__ __forceinline__ void optic_row(const OpticK& k, int s, int row, bool on, int f, const float* dr_in, float* dr_out,
+                                          Product product) {
+  constexpr bool EARLY = W * NV <= 2;
+  float y[W * NV];
+  UnitIn<W> in[EARLY ? NV : 1];
+  if constexpr (EARLY) {
 #pragma unroll
-    for (int q = 0; q < FPL; ++q) {
-      const int bb = sl * FPL + q;
-      if (bb < k.batch) optic_update(k, s, (size_t)row * k.batch + bb, row, y[q], dr_in, dr_out);
+    for (int v = 0; v < NV; ++v) {
+      const int fly = Flies<W, NV, F>::at(f, v);
+      if (on && fly < k.batch) load_unit<W>(k, (size_t)row * k.batch + fly, dr_in, in[v]);
     }
+  }
+  product(y);
+  if (!on) return;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int fly = Flies<W, NV, F>::at(f, v);
+    if (fly >= k.batch) continue;
+    const size_t t = (size_t)row * k.batch + fly;
+    if constexpr (!EARLY) load_unit<W>(k, t, dr_in, in[0]);
+    update_unit<W>(k, s, t, row, &y[v * W], in[EARLY ? v : 0], dr_out);
   }
 }
 
-template <int F, int FPL, int LPR>
+template <int LPR>
 struct OpticShape {
   static constexpr int RPW = 32 / LPR;           // row slots per warp
   static constexpr int SLOTS = 8 * RPW;          // row slots per 256-thread block
-  static constexpr int RED = SLOTS * F * FPL;    // floats of the long-row reduction
 };
 
 // Number of block work items of one substep: one per long row, then blocks of SLOTS short rows.
-template <int F, int FPL, int LPR>
+template <int LPR>
 __host__ __device__ __forceinline__ long long optic_items(int m, int n_long) {
-  constexpr int SLOTS = OpticShape<F, FPL, LPR>::SLOTS;
+  constexpr int SLOTS = OpticShape<LPR>::SLOTS;
   return n_long + (m - n_long + SLOTS - 1) / SLOTS;
 }
 
@@ -218,37 +231,37 @@ __host__ __device__ __forceinline__ long long optic_items(int m, int n_long) {
 // interleaved share of the row's entries, the shares are summed in slot order through shared
 // memory and the first slot applies the update; the longest rows thus stop bounding the substep.
 // Other rows: one row per slot.
-template <int F, int FPL, int LPR, int U>
+template <int W, int NV, int F, int LPR, int U>
 __device__ __forceinline__ void optic_item(const OpticK& k, int s, const float* dr_in, float* dr_out, long long item,
                                            float* red) {
-  using S = OpticShape<F, FPL, LPR>;
+  using S = OpticShape<LPR>;
+  constexpr int FPL = W * NV;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = lane / LPR, sl = lane % LPR;
   const int gslot = warp * S::RPW + slot;
-  float acc[FPL];
   if (item < k.n_long) {
     const int row = k.rows[item];
-    row_product<F, FPL, LPR, U>(k.ptr, k.cw, dr_in, k.batch, row, true, acc, gslot, S::SLOTS);
-    if (sl < F) {
+    const bool mine = gslot == 0 && sl < F;
+    optic_row<W, NV, F>(k, s, row, mine, sl, dr_in, dr_out, [&](float (&y)[FPL]) {
+      row_product<W, NV, F, LPR, U>(k.cw, dr_in, k.batch, __ldg(&k.ptr[row]), __ldg(&k.ptr[row + 1]), y, gslot, S::SLOTS);
+      if (sl < F) {
 #pragma unroll
-      for (int q = 0; q < FPL; ++q) red[gslot * F * FPL + sl * FPL + q] = acc[q];
-    }
-    __syncthreads();
-    if (gslot == 0 && sl < F) {
-      float y[FPL];
-#pragma unroll
-      for (int q = 0; q < FPL; ++q) y[q] = red[sl * FPL + q];
+        for (int q = 0; q < FPL; ++q) red[(gslot * F + sl) * FPL + q] = y[q];
+      }
+      __syncthreads();
+      if (!mine) return;
       for (int p = 1; p < S::SLOTS; ++p)
 #pragma unroll
-        for (int q = 0; q < FPL; ++q) y[q] = y[q] + red[p * F * FPL + sl * FPL + q];
-      optic_epilogue<F, FPL>(k, s, row, sl, y, dr_in, dr_out);
-    }
+        for (int q = 0; q < FPL; ++q) y[q] = y[q] + red[(p * F + sl) * FPL + q];
+    });
     __syncthreads();
   } else {
     const long long r = k.n_long + (item - k.n_long) * S::SLOTS + gslot;
     const bool ok = r < k.m;
     const int row = ok ? (k.rows ? k.rows[r] : (int)r) : 0;
-    row_product<F, FPL, LPR, U>(k.ptr, k.cw, dr_in, k.batch, row, ok, acc);
-    if (ok && sl < F) optic_epilogue<F, FPL>(k, s, row, sl, acc, dr_in, dr_out);
+    const int e0 = ok ? __ldg(&k.ptr[row]) : 0, e1 = ok ? __ldg(&k.ptr[row + 1]) : 0;
+    optic_row<W, NV, F>(k, s, row, ok && sl < F, sl, dr_in, dr_out, [&](float (&y)[FPL]) {
+      row_product<W, NV, F, LPR, U>(k.cw, dr_in, k.batch, e0, e1, y);
+    });
   }
 }
 
@@ -267,21 +280,22 @@ __global__ void optic_init_kernel(OpticK k) {
 
 // MINB: blocks per SM the registers must allow (launch bounds); 8 caps them at 32 per thread so a
 // full SM of 64 warps keeps gathers in flight.
-template <int F, int FPL, int LPR, int U, int MINB>
+template <int W, int NV, int F, int LPR, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) optic_step_kernel(OpticK k, int s) {
-  __shared__ float red[OpticShape<F, FPL, LPR>::RED];
+  __shared__ float red[OpticShape<LPR>::SLOTS * F * W * NV];
   const float* in = (s & 1) ? k.buf1 : k.buf0;
   float* out = (s & 1) ? k.buf0 : k.buf1;
-  optic_item<F, FPL, LPR, U>(k, s, in, out, blockIdx.x, red);
+  optic_item<W, NV, F, LPR, U>(k, s, in, out, blockIdx.x, red);
 }
 
-template <int F, int FPL, int LPR, int U, int MINB>
+template <int W, int NV, int F, int LPR, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) optic_persistent_kernel(OpticK k) {
-  __shared__ float red[OpticShape<F, FPL, LPR>::RED];
+  __shared__ float red[OpticShape<LPR>::SLOTS * F * W * NV];
+  __shared__ unsigned next;
   int generation = 0;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nth = (long long)gridDim.x * blockDim.x;
-  const long long items = optic_items<F, FPL, LPR>(k.m, k.n_long);
+  const long long items = optic_items<LPR>(k.m, k.n_long);
   if (!k.dr_valid) {
     init_dr(k, k.buf0, (int)tid, (int)nth);
     if (!grid_barrier(k.sync, k.status, generation, -1)) return;
@@ -289,12 +303,25 @@ __global__ void __launch_bounds__(256, MINB) optic_persistent_kernel(OpticK k) {
   for (int s = 0; s < k.nsteps; ++s) {
     const float* in = (s & 1) ? k.buf1 : k.buf0;
     float* out = (s & 1) ? k.buf0 : k.buf1;
-    for (long long item = blockIdx.x; item < items; item += gridDim.x) optic_item<F, FPL, LPR, U>(k, s, in, out, item, red);
+    // Items are handed out as blocks come for them (long rows first, then shorter and shorter ones):
+    // the first gridDim.x <= items by block, the others by a count in sync[1], which grows by one per
+    // item and so by `items` per substep. Thread 0 asks for the next item beside the current one.
+    // (Asking three items ahead, with the next rows' bounds on their way: 34.5 us against 32.0 at
+    // one fly, 59 against 55 at 12: the gathers, not the row bounds, are what the warps wait for.)
+    for (long long item = blockIdx.x; item < items;) {
+      unsigned given = 0;
+      if (threadIdx.x == 0) given = (unsigned)atomicAdd(&k.sync[1], 1) - (unsigned)(s * items);
+      optic_item<W, NV, F, LPR, U>(k, s, in, out, item, red);
+      if (threadIdx.x == 0) next = given;
+      __syncthreads();
+      item = (long long)gridDim.x + next;
+      __syncthreads();
+    }
     if (s + 1 < k.nsteps && !grid_barrier(k.sync, k.status, generation, s)) return;
   }
 }
 
-template <int F, int FPL, int LPR, int U = Unroll<FPL>::U, int MINB = 1>
+template <int W, int NV, int F, int LPR, int U, int MINB>
 static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st) {
   const long long sz = (long long)k.m * k.batch;
   if (launch == FLYB_LAUNCH_STEP) {
@@ -302,9 +329,9 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
       optic_init_kernel<<<(unsigned)((sz + 255) / 256), 256, 0, st>>>(k);
       FLYB_CHECK_LAUNCH();
     }
-    const unsigned blocks = (unsigned)optic_items<F, FPL, LPR>(k.m, k.n_long);
+    const unsigned blocks = (unsigned)optic_items<LPR>(k.m, k.n_long);
     for (int s = 0; s < k.nsteps; ++s) {
-      optic_step_kernel<F, FPL, LPR, U, MINB><<<blocks, 256, 0, st>>>(k, s);
+      optic_step_kernel<W, NV, F, LPR, U, MINB><<<blocks, 256, 0, st>>>(k, s);
       FLYB_CHECK_LAUNCH();
     }
     return 0;
@@ -312,41 +339,26 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, optic_persistent_kernel<F, FPL, LPR, U, MINB>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, optic_persistent_kernel<W, NV, F, LPR, U, MINB>, 256, 0);
   long long grid = (long long)sms * per_sm;
-  const long long need = optic_items<F, FPL, LPR>(k.m, k.n_long);
+  const long long need = optic_items<LPR>(k.m, k.n_long);
   if (grid > need) grid = need;
   if (grid_cap > 0 && grid > grid_cap) grid = grid_cap;
   if (grid < 1) return FLYB_ECOOP;
+  cudaError_t e = cudaMemsetAsync(k.sync, 0, 2 * sizeof(int), st);   // barrier and item counts
+  if (e != cudaSuccess) return (int)e;
   if (k.nsteps == 1 && k.dr_valid) {
     // one substep on a carried dr reaches no grid barrier: an ordinary launch of `grid` blocks
     // looping over the items, which other kernels may share the SMs with
-    optic_persistent_kernel<F, FPL, LPR, U, MINB><<<(unsigned)grid, 256, 0, st>>>(k);
+    optic_persistent_kernel<W, NV, F, LPR, U, MINB><<<(unsigned)grid, 256, 0, st>>>(k);
     return (int)cudaGetLastError();
   }
-  cudaError_t e = cudaMemsetAsync(k.sync, 0, 2 * sizeof(int), st);
-  if (e != cudaSuccess) return (int)e;
   OpticK kk = k;
   void* args[] = {&kk};
-  e = cudaLaunchCooperativeKernel((void*)optic_persistent_kernel<F, FPL, LPR, U, MINB>, dim3((unsigned)grid), dim3(256), args, 0,
+  e = cudaLaunchCooperativeKernel((void*)optic_persistent_kernel<W, NV, F, LPR, U, MINB>, dim3((unsigned)grid), dim3(256), args, 0,
                                   st);
   return (int)e;
 }
-
-// Picks (F, FPL) from the batch: F lanes across flies, FPL consecutive flies per lane.
-#define FLYB_BATCH_DISPATCH(B, CALL)                                   \
-  do {                                                                 \
-    if ((B) == 1) { constexpr int F = 1, FPL = 1; return CALL; }       \
-    if ((B) <= 2) { constexpr int F = 2, FPL = 1; return CALL; }       \
-    if ((B) <= 4) { constexpr int F = 4, FPL = 1; return CALL; }       \
-    if ((B) <= 8) { constexpr int F = 8, FPL = 1; return CALL; }       \
-    if ((B) <= 16) { constexpr int F = 16, FPL = 1; return CALL; }     \
-    if ((B) <= 32) { constexpr int F = 32, FPL = 1; return CALL; }     \
-    if ((B) <= 64) { constexpr int F = 32, FPL = 2; return CALL; }     \
-    if ((B) <= 128) { constexpr int F = 32, FPL = 4; return CALL; }    \
-    if ((B) <= 256) { constexpr int F = 32, FPL = 8; return CALL; }    \
-    return FLYB_ETOOBIG;                                               \
-  } while (0)
 
 // (F fly lanes, FPL flies per lane) of the held-input products: from 32 flies on, 4 flies per lane
 // so that a warp instruction covers 2-4 entries (the per-entry index and weight work is shared by
@@ -365,50 +377,92 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
     return FLYB_ETOOBIG;                                               \
   } while (0)
 
-// (F fly lanes, FPL flies per lane, LPR lanes per row, U gathers in flight per lane, MINB blocks per
-// SM) of the optic substep for a batch; `variant` 0 is the default, the others are alternatives the
-// autotuner tries (more warps with fewer registers each, or wider lanes); an unknown variant is an
-// error.
-#define FLYB_OPTIC_DISPATCH(B, V, CALL)                                                           \
-  do {                                                                                            \
-    if ((B) == 1) {                                                                               \
-      if ((V) == 0) { constexpr int F = 1, FPL = 1, LPR = 8, U = 8, MINB = 1; return CALL; }      \
-      if ((V) == 1) { constexpr int F = 1, FPL = 1, LPR = 16, U = 8, MINB = 1; return CALL; }     \
-      if ((V) == 2) { constexpr int F = 1, FPL = 1, LPR = 32, U = 8, MINB = 1; return CALL; }     \
-      if ((V) == 3) { constexpr int F = 1, FPL = 1, LPR = 8, U = 4, MINB = 8; return CALL; }      \
-      if ((V) == 4) { constexpr int F = 1, FPL = 1, LPR = 16, U = 4, MINB = 8; return CALL; }     \
-      return FLYB_EINVAL;                                                                         \
-    }                                                                                             \
-    if ((V) != 0 && (B) <= 32) return FLYB_EINVAL;                                                \
-    if ((B) <= 2) { constexpr int F = 2, FPL = 1, LPR = 16, U = 8, MINB = 1; return CALL; }       \
-    if ((B) <= 4) { constexpr int F = 4, FPL = 1, LPR = 16, U = 8, MINB = 1; return CALL; }       \
-    if ((B) <= 8) { constexpr int F = 8, FPL = 1, LPR = 32, U = 8, MINB = 1; return CALL; }       \
-    if ((B) <= 16) { constexpr int F = 16, FPL = 1, LPR = 32, U = 8, MINB = 1; return CALL; }     \
-    if ((B) <= 32) { constexpr int F = 32, FPL = 1, LPR = 32, U = 8, MINB = 1; return CALL; }     \
-    if ((B) <= 64) {                                                                              \
-      if ((V) == 0) { constexpr int F = 16, FPL = 4, LPR = 32, U = 4, MINB = 1; return CALL; }    \
-      if ((V) == 1) { constexpr int F = 32, FPL = 2, LPR = 32, U = 8, MINB = 1; return CALL; }    \
-      if ((V) == 2) { constexpr int F = 8, FPL = 8, LPR = 32, U = 2, MINB = 1; return CALL; }     \
-      if ((V) == 3) { constexpr int F = 16, FPL = 4, LPR = 32, U = 2, MINB = 8; return CALL; }    \
-      if ((V) == 4) { constexpr int F = 32, FPL = 2, LPR = 32, U = 4, MINB = 8; return CALL; }    \
-      if ((V) == 5) { constexpr int F = 16, FPL = 4, LPR = 32, U = 4, MINB = 6; return CALL; }    \
-      return FLYB_EINVAL;                                                                         \
-    }                                                                                             \
-    if ((B) <= 128) {                                                                             \
-      if ((V) == 0) { constexpr int F = 32, FPL = 4, LPR = 32, U = 4, MINB = 1; return CALL; }    \
-      if ((V) == 1) { constexpr int F = 16, FPL = 8, LPR = 32, U = 2, MINB = 1; return CALL; }    \
-      if ((V) == 3) { constexpr int F = 32, FPL = 4, LPR = 32, U = 2, MINB = 8; return CALL; }    \
-      return FLYB_EINVAL;                                                                         \
-    }                                                                                             \
-    if ((B) <= 256) {                                                                             \
-      if ((V) == 0) { constexpr int F = 32, FPL = 8, LPR = 32, U = 2, MINB = 1; return CALL; }    \
-      if ((V) == 1) { constexpr int F = 32, FPL = 8, LPR = 32, U = 2, MINB = 4; return CALL; }    \
-      if ((V) == 3) { constexpr int F = 32, FPL = 8, LPR = 32, U = 1, MINB = 6; return CALL; }    \
-      if ((V) == 5) { constexpr int F = 32, FPL = 8, LPR = 32, U = 1, MINB = 8; return CALL; }    \
-      return FLYB_EINVAL;                                                                         \
-    }                                                                                             \
-    return FLYB_ETOOBIG;                                                                          \
-  } while (0)
+// Widest vector access the batch and the arrays allow: W flies, W dividing the batch and every array
+// W floats aligned.
+static int vector_width(const OpticK& k) {
+  const void* arrays[] = {k.v, k.adapt, k.buf0, k.buf1, k.pr, k.spk, k.v_hist, k.inp_hist};
+  for (int w = 4; w > 1; w >>= 1) {
+    bool ok = k.batch % w == 0;
+    for (const void* p : arrays) ok = ok && (reinterpret_cast<uintptr_t>(p) & (4 * w - 1)) == 0;
+    if (ok) return w;
+  }
+  return 1;
+}
+
+// The substep's kernel shape for a batch, k.batch <= 256. Variant 0: vectors as wide as the batch
+// allows, spread over the fewest fly lanes, so that a warp instruction gathers for as many entries
+// as it can: the gathers then run at the L2's rate instead of the issue rate (89,390 units, 6 M
+// entries, one substep: 12 flies 162 us with 16 lanes of one fly, 55 us with 4 lanes of four; 24
+// flies 294 -> 80; 64 flies 254 -> 115 us and 128 flies 416 -> 254 us with the registers bounded for
+// six and four blocks per SM). Narrow rows leave lanes over for entries; a
+// lobe of few rows gives each row a whole warp (LPR 32), so that its rows still fill the SMs. The
+// other variants are what the autotuner tries beside it; one that the vector width rules out runs
+// as variant 0, an unknown one is an error.
+static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cudaStream_t st) {
+  const int B = k.batch, w = vector_width(k);
+  const bool few = k.m <= 148 * 64;          // rows that a warp each would still hold on the SMs
+#define FLYB_RUN(...) return run_optic<__VA_ARGS__>(k, launch, cap, st)
+  if (B > 256) return FLYB_ETOOBIG;
+  if (variant < 0 || variant > 5) return FLYB_EINVAL;
+  if (B == 1) {
+    switch (variant) {
+      case 0: if (few) FLYB_RUN(1, 1, 1, 32, 4, 4); else FLYB_RUN(1, 1, 1, 8, 8, 4);
+      case 1: FLYB_RUN(1, 1, 1, 16, 8, 1);
+      case 2: FLYB_RUN(1, 1, 1, 32, 8, 1);
+      case 3: FLYB_RUN(1, 1, 1, 8, 4, 8);
+      case 4: FLYB_RUN(1, 1, 1, 16, 4, 8);
+      default: return FLYB_EINVAL;
+    }
+  }
+  if (variant && B <= 32) return FLYB_EINVAL;
+  if (B > 32 && B <= 64 && variant) {
+    if (w == 4 && variant == 2) FLYB_RUN(4, 2, 8, 32, 2, 3);
+    if (w == 4 && variant == 3) FLYB_RUN(4, 1, 16, 32, 2, 8);
+    if (w == 4 && variant == 5) FLYB_RUN(4, 1, 16, 32, 4, 4);
+    if (w >= 2 && variant == 1) FLYB_RUN(2, 1, 32, 32, 8, 4);
+    if (w >= 2 && variant == 4) FLYB_RUN(2, 1, 32, 32, 4, 8);
+  }
+  if (B > 64 && B <= 128 && variant) {
+    if (variant != 1 && variant != 3) return FLYB_EINVAL;
+    if (w == 4 && variant == 1) FLYB_RUN(4, 2, 16, 32, 2, 3);
+    if (w == 4 && variant == 3) FLYB_RUN(4, 1, 32, 32, 2, 8);
+  }
+  if (B > 128 && variant) {
+    if (variant != 1 && variant != 3 && variant != 5) return FLYB_EINVAL;
+    if (w == 4 && variant == 1) FLYB_RUN(4, 2, 32, 32, 2, 1);
+    if (w == 4 && variant == 3) FLYB_RUN(4, 2, 32, 32, 1, 6);
+    if (w == 4 && variant == 5) FLYB_RUN(4, 2, 32, 32, 1, 8);
+  }
+  const int vectors = B / w;
+  if (w == 4) {
+    if (vectors == 1) { if (few) FLYB_RUN(4, 1, 1, 32, 2, 4); else FLYB_RUN(4, 1, 1, 8, 4, 4); }
+    if (vectors == 2) { if (few) FLYB_RUN(4, 1, 2, 32, 4, 4); else FLYB_RUN(4, 1, 2, 16, 4, 4); }
+    if (vectors <= 4) FLYB_RUN(4, 1, 4, 32, 4, 5);
+    if (vectors <= 8) FLYB_RUN(4, 1, 8, 32, 4, 5);
+    if (vectors <= 16) FLYB_RUN(4, 1, 16, 32, 4, 6);
+    if (vectors <= 32) FLYB_RUN(4, 1, 32, 32, 4, 4);
+    FLYB_RUN(4, 2, 32, 32, 2, 4);
+  }
+  if (w == 2) {
+    if (vectors == 1) { if (few) FLYB_RUN(2, 1, 1, 32, 4, 4); else FLYB_RUN(2, 1, 1, 8, 8, 4); }
+    if (vectors == 2) FLYB_RUN(2, 1, 2, 16, 8, 4);
+    if (vectors <= 4) FLYB_RUN(2, 1, 4, 32, 4, 5);
+    if (vectors <= 8) FLYB_RUN(2, 1, 8, 32, 8, 4);
+    if (vectors <= 16) FLYB_RUN(2, 1, 16, 32, 8, 4);
+    if (vectors <= 32) FLYB_RUN(2, 1, 32, 32, 8, 4);
+    if (vectors <= 64) FLYB_RUN(2, 2, 32, 32, 4, 4);
+    FLYB_RUN(2, 4, 32, 32, 2, 4);
+  }
+  if (B == 2) FLYB_RUN(1, 1, 2, 16, 8, 4);
+  if (B <= 4) FLYB_RUN(1, 1, 4, 32, 8, 4);
+  if (B <= 8) FLYB_RUN(1, 1, 8, 32, 8, 4);
+  if (B <= 16) FLYB_RUN(1, 1, 16, 32, 8, 4);
+  if (B <= 32) FLYB_RUN(1, 1, 32, 32, 8, 4);
+  if (B <= 64) FLYB_RUN(1, 2, 32, 32, 4, 5);
+  if (B <= 128) FLYB_RUN(1, 4, 32, 32, 4, 4);
+  FLYB_RUN(1, 8, 32, 32, 2, 4);
+#undef FLYB_RUN
+}
 
 // ------------------------------------------------------------------ held-input products
 struct SpmmK {
@@ -584,7 +638,7 @@ __global__ void ref_csr_kernel(const int* __restrict__ ptr, const int* __restric
 
 int optic_blocks_per_sm() {
   int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, optic_persistent_kernel<1, 1, 8, 8, 1>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, optic_persistent_kernel<1, 1, 1, 8, 8, 4>, 256, 0);
   return b;
 }
 
@@ -606,7 +660,7 @@ FLYB_API int flyb_optic_run(const flyb_optic_args* a, void* stream) {
            (a->flags & FLYB_OPTIC_HISTORY) ? a->inp_hist : nullptr, a->status, a->sync,
            (a->flags & FLYB_OPTIC_DR_VALID) ? 1 : 0};
   cudaStream_t st = (cudaStream_t)stream;
-  FLYB_OPTIC_DISPATCH(a->batch, a->variant, (run_optic<F, FPL, LPR, U, MINB>(k, a->launch, a->grid, st)));
+  return run_optic_shape(k, a->variant, a->launch, a->grid, st);
 }
 
 // ------------------------------------------------------------------ allocation-free variant
@@ -654,7 +708,7 @@ FLYB_API int flyb_optic_run_noalloc(const flyb_optic_args* a, void* stream) {
            (a->flags & FLYB_OPTIC_HISTORY) ? a->inp_hist : nullptr, a->status,
            (int*)(scratch + 2 * FLYB_OPTIC_NOALLOC_MAX), 0};
   cudaStream_t st = (cudaStream_t)stream;
-  FLYB_OPTIC_DISPATCH(a->batch, a->variant, (run_optic<F, FPL, LPR, U, MINB>(k, a->launch, a->grid, st)));
+  return run_optic_shape(k, a->variant, a->launch, a->grid, st);
 }
 
 FLYB_API int flyb_spmm(const flyb_spmm_args* a, void* stream) {

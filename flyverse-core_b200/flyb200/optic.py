@@ -164,7 +164,14 @@ def spmm(M: DeviceCSR, x: torch.Tensor, y: torch.Tensor, *, x_index=None, x_div=
         raise RuntimeError(f"flyb_spmm: error {rc}")
 
 
-LONG_ROW = 192      # rows with more entries than this are split across a whole block
+def long_row_entries(nnz: int, sms: int = 148) -> int:
+    """Entries above which a row is split across a whole block (OpticCore.set_long_rows): three times
+    the entries that each of the ~48 resident warps per SM has to itself, between 96 and 512. A large
+    lobe has work enough that only the longest rows hold it up, and splitting costs a block's
+    reduction; in a small one a warp's single row may last as long as the whole substep. Measured
+    per substep at thresholds 192 / 512: 6 M entries 44.9 / 34.8 us at one fly and 121 / 115 at 64;
+    at 96 / 192: 0.1 M entries 8.5 / 12.6 us at 64 flies."""
+    return max(96, min(512, 3 * nnz // (48 * sms)))
 
 
 class OpticCore:
@@ -198,7 +205,7 @@ class OpticCore:
         self.launch = launch
         self.variant = 0                 # kernel shape (flyb_optic_args.variant), set by the autotuner
         self.grid = 0                    # persistent launches: block cap (0 = every resident block)
-        self.set_long_rows(LONG_ROW)
+        self.set_long_rows(long_row_entries(self.W.nnz, _sm_count(self.device)))
         M, B, dev = self.m, self.B, self.device
         self.v_s = torch.zeros(M, B, device=dev)
         self.adapt_s = torch.zeros(M, B, device=dev)

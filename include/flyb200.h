@@ -282,7 +282,8 @@ typedef struct flyb_optic_args {
   int launch;            /* FLYB_LAUNCH_*                                            */
   int block;             /* threads per block (0 = default)                          */
   int grid;              /* persistent grid cap (0 = occupancy)                      */
-  int variant;           /* kernel shape: 0 default, 1 / 2 alternatives (autotuned)  */
+  int variant;           /* kernel shape: 0 the rule's choice for the batch, 1-5 alternatives
+                            (autotuned; at one fly and above 32)                     */
   int flags;             /* FLYB_OPTIC_*                                             */
   const int* ptr;        /* W_rr CSR row pointers [m + 1], rows = postsynaptic units */
   const int* cw;         /* [nnz][2] interleaved {column, float bits of weight}      */
