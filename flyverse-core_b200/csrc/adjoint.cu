@@ -13,10 +13,15 @@
 //   dL/dad_t  = aad * lam_a - ga * mu_t
 //   g_edge[e] += mu_t[i] * dr_t[j]        for e = (i <- j): dL/dW_ij = gr * g_edge[e]
 //   g_a[i]    += lam_v[i] * (v_t[i] - inp_t[i])   (dL/da_i)
-// W^T is walked as the CSR of the transpose: warp w owns transposed rows j (presynaptic units),
+// W^T is walked as the CSR of the transpose: a row slot owns a transposed row j (presynaptic unit),
 // so the per-edge accumulator g_edge, g_a[j] and the in-place lam updates of row j have a single
-// writer. mu is double-buffered, so one grid barrier per reverse step suffices.
-#include "common.cuh"
+// writer. With lam of step t - 1 in hand the slot goes on to mu_{t-1} and the g_a term of its
+// unit, so a reverse step is one pass over the rows and, mu being double-buffered, one grid
+// barrier. Bound: the entries with their accumulator (16 bytes per edge and step) and the gathers of
+// mu, both out of L2. Measured per reverse step: 89,390 units, 6 M entries, one fly 63 -> 52 us; 20,000
+// units, 1.34 M entries, 16 flies 85 -> 25 us (four lanes of four flies instead of sixteen of one;
+// the per-edge sums by halving exchanges).
+#include "flies.cuh"
 
 namespace flyb {
 
@@ -33,155 +38,253 @@ struct AdjK {
   int* status; int* sync;
 };
 
-// Phase 1 for the rows of this warp: mu_t = (1 - a) lam_v and the g_a accumulation.
-template <int F, int FPL>
-__device__ __forceinline__ void adj_phase1(const AdjK& k, int t, float* mu, long long warp0, long long nwarps) {
-  const int lane = threadIdx.x & 31;
-  const size_t sz = (size_t)k.m * k.batch;
-  for (long long j = warp0; j < k.m; j += nwarps) {
-    float part = 0.0f;
-    if (lane < F) {
-      const float aj = k.a[j];
-      const float oma = 1.0f - aj;
+// mu_t = (1 - a) lam_v of unit j on the slot's fly lanes, and its g_a term of step t.
+template <int W, int NV, int F>
+__device__ __forceinline__ void adj_unit(const AdjK& k, int t, int j, bool on, int sl, const float* lam, float* mu) {
+  const size_t at = (size_t)t * ((size_t)k.m * k.batch);
+  float part = 0.0f;
+  if (on) {
+    const float oma = 1.0f - k.a[j];
 #pragma unroll
-      for (int q = 0; q < FPL; ++q) {
-        const int bb = lane * FPL + q;
-        if (bb < k.batch) {
-          const size_t e = (size_t)j * k.batch + bb;
-          const float lv = k.lam_v[e];
-          mu[e] = oma * lv;
-          const float d = k.v_hist[(size_t)t * sz + e] - k.inp_hist[(size_t)t * sz + e];
-          part = part + lv * d;
-        }
+    for (int v = 0; v < NV; ++v) {
+      const int fly = Flies<W, NV, F>::at(sl, v);
+      if (fly >= k.batch) continue;
+      const size_t e = (size_t)j * k.batch + fly;
+      float x[W], y[W], m[W];
+      load_w<W>(k.v_hist + at + e, x);
+      load_w<W>(k.inp_hist + at + e, y);
+#pragma unroll
+      for (int q = 0; q < W; ++q) {
+        m[q] = oma * lam[v * W + q];
+        part = fmaf(lam[v * W + q], x[q] - y[q], part);
       }
+      store_w<W>(mu + e, m);
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) part = part + __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) k.g_a[j] = k.g_a[j] + part;
   }
+#pragma unroll
+  for (int o = 1; o < F; o <<= 1) part = part + __shfl_xor_sync(0xffffffffu, part, o);
+  if (on && sl == 0) k.g_a[j] = k.g_a[j] + part;
 }
 
-// Phase 2: z = W^T mu over transposed row j, the lam updates and the per-edge accumulation.
-template <int F, int FPL>
-__device__ __forceinline__ void adj_phase2(const AdjK& k, int t, const float* __restrict__ mu, long long warp0,
-                                           long long nwarps) {
-  constexpr int G = 32 / F;
-  const int lane = threadIdx.x & 31, g = lane / F, f = lane % F, fb = f * FPL;
-  const size_t sz = (size_t)k.m * k.batch;
-  for (long long j = warp0; j < k.m; j += nwarps) {
-    const float bj = k.b[j];
-    float dr[FPL];
+// Sums ge[u], u < U, over the F fly lanes of the group and adds them to the accumulators of the
+// entries base + u * stride. While two or more entries are left a halving exchange leaves each
+// half of the lanes with half of the entries (U = 4, F = 16: 5 exchanges instead of 16); the
+// remaining exchanges sum whole.
+template <int F, int U>
+__device__ __forceinline__ void add_edges(const AdjK& k, float (&ge)[U], int base, int stride, int e1, int f) {
+  int first = 0;
+  int left = U;
 #pragma unroll
-    for (int q = 0; q < FPL; ++q) {
-      const int bb = fb + q;
-      dr[q] = bb < k.batch ? clip01(k.v_hist[(size_t)t * sz + (size_t)j * k.batch + bb] + bj) - bj : 0.0f;
+  for (int o = F / 2, n = U; o >= 1; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = f & o;
+#pragma unroll
+      for (int q = 0; q < U / 2; ++q)
+        if (q < n) {
+          const float send = up ? ge[q] : ge[q + n], keep = up ? ge[q + n] : ge[q];
+          ge[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      first += up ? n : 0;
+      left = n;
+    } else {
+      ge[0] = ge[0] + __shfl_xor_sync(0xffffffffu, ge[0], o);
     }
-    float acc[FPL];
+  }
+  // lanes that hold the same sums: the one whose remaining lane bits are zero writes
+  constexpr int SAME = F > U ? F / U : 1;
+  if (f & (SAME - 1)) return;
 #pragma unroll
-    for (int q = 0; q < FPL; ++q) acc[q] = 0.0f;
-    constexpr int U = FPL <= 2 ? 8 : (FPL == 4 ? 4 : 2);
-    const int e0 = k.t_ptr[j], e1 = k.t_ptr[j + 1];
-    // lane group g takes entries e0 + g + G*k; U gathers of mu in flight per lane
-    for (int base = e0 + g; base - g < e1; base += G * U) {
-      int ii[U];
-      float ww[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int e = base + u * G;
-        const bool ok = e < e1;
-        ii[u] = ok ? __ldg(&k.t_col[e]) : -1;
-        ww[u] = ok ? __ldg(&k.t_w[e]) : 0.0f;
-      }
-      float mv[U][FPL];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int q = 0; q < FPL; ++q)
-          mv[u][q] = (ii[u] >= 0 && fb + q < k.batch) ? mu[(size_t)ii[u] * k.batch + fb + q] : 0.0f;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        float ge = 0.0f;
-#pragma unroll
-        for (int q = 0; q < FPL; ++q) {
-          const float p = ww[u] * mv[u][q];
-          acc[q] = acc[q] + p;
-          const float pg = mv[u][q] * dr[q];
-          ge = ge + pg;
-        }
-        // sum the per-edge term over the F lanes of this group (every lane takes part)
-#pragma unroll
-        for (int o = 1; o < F; o <<= 1) ge = ge + __shfl_xor_sync(0xffffffffu, ge, o);
-        if (ii[u] >= 0 && f == 0) {
-          const int ee = base + u * G;
-          const int pe = k.t_perm ? k.t_perm[ee] : ee;
-          k.g_edge[pe] = k.g_edge[pe] + ge;
-        }
-      }
-    }
-#pragma unroll
-    for (int o = F; o < 32; o <<= 1)
-#pragma unroll
-      for (int q = 0; q < FPL; ++q) acc[q] = acc[q] + __shfl_xor_sync(0xffffffffu, acc[q], o);
-    if (lane < F) {
-      const float aj = k.a[j];
-      const float omaad = 1.0f - k.aad;
-#pragma unroll
-      for (int q = 0; q < FPL; ++q) {
-        const int bb = lane * FPL + q;
-        if (bb < k.batch) {
-          const size_t e = (size_t)j * k.batch + bb;
-          const float x = k.v_hist[(size_t)t * sz + e] + bj;
-          const float mask = (x >= 0.0f && x <= 1.0f) ? 1.0f : 0.0f;
-          const float lv = k.lam_v[e], la = k.lam_a[e];
-          float inner = k.gr * acc[q];
-          inner = inner + omaad * la;
-          float nl = aj * lv;
-          nl = nl + mask * inner;
-          k.lam_v[e] = nl;
-          float na = k.aad * la;
-          na = na - k.ga * mu[e];
-          k.lam_a[e] = na;
-        }
-      }
+  for (int q = 0; q < U; ++q) {
+    const int e = base + (first + q) * stride;
+    if (q < left && e < e1) {
+      const int pe = k.t_perm ? k.t_perm[e] : e;
+      k.g_edge[pe] = k.g_edge[pe] + ge[q];
     }
   }
 }
 
-template <int F, int FPL>
-__global__ void __launch_bounds__(256) adj_phase1_kernel(AdjK k, int t) {
-  float* mu = (t & 1) ? k.mu1 : k.mu0;
-  adj_phase1<F, FPL>(k, t, mu, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                     ((long long)gridDim.x * blockDim.x) >> 5);
+// Entries [e0, e1) of transposed row j on a slot of LPR lanes: acc += W^T mu of the lane's flies (complete
+// on slot lanes < F), and the edges' accumulators.
+template <int W, int NV, int F, int LPR, int U>
+__device__ __forceinline__ void adj_entries(const AdjK& k, const float* mu, int e0, int e1, const float (&dr)[W * NV],
+                                            float (&acc)[W * NV]) {
+  constexpr int G = LPR / F, FPL = W * NV;
+  const int sl = (threadIdx.x & 31) % LPR, g = sl / F, f = sl % F;
+  const float* ml[NV];
+  bool in[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int fly = Flies<W, NV, F>::at(f, v);
+    in[v] = fly < k.batch;
+    ml[v] = mu + (in[v] ? fly : 0);
+  }
+#pragma unroll
+  for (int q = 0; q < FPL; ++q) acc[q] = 0.0f;
+  // every lane of the warp takes part in the exchanges: the slots go on to the longest one's end
+  const int trips = __reduce_max_sync(0xffffffffu, (e1 - e0 + G * U - 1) / (G * U));
+  for (int trip = 0, base = e0 + g; trip < trips; ++trip, base += G * U) {
+    int ii[U];
+    float ww[U], mv[U][FPL], ge[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = base + u * G;
+      const bool ok = e < e1;
+      ii[u] = ok ? __ldg(&k.t_col[e]) : 0;
+      ww[u] = ok ? __ldg(&k.t_w[e]) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) load_w<W>(ml[v] + (size_t)ii[u] * k.batch, &mv[u][v * W]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = base + u * G < e1;
+      ge[u] = 0.0f;
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int q = v * W; q < (v + 1) * W; ++q) {
+          const float m = ok && in[v] ? mv[u][q] : 0.0f;
+          acc[q] = fmaf(ww[u], m, acc[q]);
+          ge[u] = fmaf(m, dr[q], ge[u]);
+        }
+    }
+    add_edges<F, U>(k, ge, base, G, e1, f);
+  }
+#pragma unroll
+  for (int o = F; o < LPR; o <<= 1)
+#pragma unroll
+    for (int q = 0; q < FPL; ++q) acc[q] = acc[q] + __shfl_xor_sync(0xffffffffu, acc[q], o);
 }
 
-template <int F, int FPL>
-__global__ void __launch_bounds__(256) adj_phase2_kernel(AdjK k, int t) {
-  const float* mu = (t & 1) ? k.mu1 : k.mu0;
-  adj_phase2<F, FPL>(k, t, mu, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                     ((long long)gridDim.x * blockDim.x) >> 5);
+// Step t for the transposed row of each slot: z = W^T mu_t, the per-edge accumulation, lam of step
+// t - 1 in place, then mu_{t-1} and g_a (t > 0). Rows of more than kAdjWide entries are left by
+// narrow slots to the whole warp, one after the other.
+constexpr int kAdjWide = 512;
+
+template <int W, int NV, int F, int LPR, int U>
+__device__ __forceinline__ void adj_item(const AdjK& k, int t, const float* mu, float* mu_next, long long item) {
+  using S = RowSlots<LPR>;
+  constexpr int FPL = W * NV;
+  const int lane = threadIdx.x & 31, sl = lane % LPR, f = sl % F;
+  const long long r = item * S::SLOTS + (threadIdx.x >> 5) * S::RPW + lane / LPR;
+  const bool ok = r < k.m;
+  const int j = ok ? (int)r : k.m - 1;
+  const size_t sz = (size_t)k.m * k.batch, at = (size_t)t * sz;
+  int e0 = 0, e1 = 0;
+  if (ok) { e0 = __ldg(&k.t_ptr[j]); e1 = __ldg(&k.t_ptr[j + 1]); }
+  const float bj = k.b[j];
+  float x[FPL], dr[FPL], acc[FPL];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int fly = Flies<W, NV, F>::at(f, v);
+    load_w<W>(k.v_hist + at + (size_t)j * k.batch + (fly < k.batch ? fly : 0), &x[v * W]);
+  }
+#pragma unroll
+  for (int q = 0; q < FPL; ++q) {
+    x[q] = x[q] + bj;
+    dr[q] = clip01(x[q]) - bj;
+  }
+  const bool wide = LPR < 32 && e1 - e0 > kAdjWide;
+  adj_entries<W, NV, F, LPR, U>(k, mu, e0, wide ? e0 : e1, dr, acc);
+  if constexpr (LPR < 32) {
+    for (unsigned todo = __ballot_sync(0xffffffffu, wide && sl == 0); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;                         // first lane of the slot
+      const int w0 = __shfl_sync(0xffffffffu, e0, src), w1 = __shfl_sync(0xffffffffu, e1, src);
+      float wdr[FPL], wacc[FPL];
+#pragma unroll
+      for (int q = 0; q < FPL; ++q) wdr[q] = __shfl_sync(0xffffffffu, dr[q], src + lane % F);
+      adj_entries<W, NV, F, 32, U>(k, mu, w0, w1, wdr, wacc);  // complete on lanes < F
+#pragma unroll
+      for (int q = 0; q < FPL; ++q) {
+        const float got = __shfl_sync(0xffffffffu, wacc[q], f);
+        if (lane - sl == src) acc[q] = got;
+      }
+    }
+  }
+  const bool on = ok && sl < F;
+  float nl[FPL];
+#pragma unroll
+  for (int q = 0; q < FPL; ++q) nl[q] = 0.0f;
+  if (on) {
+    const float aj = k.a[j], omaad = 1.0f - k.aad;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int fly = Flies<W, NV, F>::at(sl, v);
+      if (fly >= k.batch) continue;
+      const size_t e = (size_t)j * k.batch + fly;
+      float lv[W], la[W], m[W], na[W];
+      load_w<W>(k.lam_v + e, lv);
+      load_w<W>(k.lam_a + e, la);
+      load_w<W>(mu + e, m);
+#pragma unroll
+      for (int q = 0; q < W; ++q) {
+        const float mask = (x[v * W + q] >= 0.0f && x[v * W + q] <= 1.0f) ? 1.0f : 0.0f;
+        float inner = k.gr * acc[v * W + q];
+        inner = inner + omaad * la[q];
+        nl[v * W + q] = aj * lv[q];
+        nl[v * W + q] = nl[v * W + q] + mask * inner;
+        na[q] = k.aad * la[q];
+        na[q] = na[q] - k.ga * m[q];
+      }
+      store_w<W>(k.lam_v + e, &nl[v * W]);
+      store_w<W>(k.lam_a + e, na);
+    }
+  }
+  if (t > 0) adj_unit<W, NV, F>(k, t - 1, j, on, sl, nl, mu_next);
 }
 
-template <int F, int FPL>
-__global__ void __launch_bounds__(256) adj_persistent_kernel(AdjK k) {
+// mu and g_a of the last step of the segment, from the given lam.
+template <int W, int NV, int F, int LPR>
+__device__ __forceinline__ void adj_first_item(const AdjK& k, long long item) {
+  using S = RowSlots<LPR>;
+  const int lane = threadIdx.x & 31, sl = lane % LPR;
+  const long long r = item * S::SLOTS + (threadIdx.x >> 5) * S::RPW + lane / LPR;
+  const bool on = r < k.m && sl < F;
+  const int j = r < k.m ? (int)r : k.m - 1, t = k.nsteps - 1;
+  float lam[W * NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int fly = Flies<W, NV, F>::at(sl % F, v);
+    load_w<W>(k.lam_v + (size_t)j * k.batch + (fly < k.batch ? fly : 0), &lam[v * W]);
+  }
+  adj_unit<W, NV, F>(k, t, j, on, sl, lam, (t & 1) ? k.mu1 : k.mu0);
+}
+
+template <int W, int NV, int F, int LPR, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) adj_first_kernel(AdjK k) {
+  adj_first_item<W, NV, F, LPR>(k, blockIdx.x);
+}
+
+template <int W, int NV, int F, int LPR, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) adj_step_kernel(AdjK k, int t) {
+  adj_item<W, NV, F, LPR, U>(k, t, (t & 1) ? k.mu1 : k.mu0, (t & 1) ? k.mu0 : k.mu1, blockIdx.x);
+}
+
+template <int W, int NV, int F, int LPR, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) adj_persistent_kernel(AdjK k) {
+  __shared__ unsigned next;
   int generation = 0;
-  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long items = (k.m + RowSlots<LPR>::SLOTS - 1) / RowSlots<LPR>::SLOTS;
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) adj_first_item<W, NV, F, LPR>(k, item);
   for (int t = k.nsteps - 1; t >= 0; --t) {
-    float* mu = (t & 1) ? k.mu1 : k.mu0;
-    adj_phase1<F, FPL>(k, t, mu, w0, nw);
     if (!grid_barrier(k.sync, k.status, generation, t)) return;
-    adj_phase2<F, FPL>(k, t, mu, w0, nw);
+    const float* mu = (t & 1) ? k.mu1 : k.mu0;
+    float* mu_next = (t & 1) ? k.mu0 : k.mu1;
+    deal_items(&k.sync[1], (unsigned)(k.nsteps - 1 - t), items, &next,
+               [&](long long item) { adj_item<W, NV, F, LPR, U>(k, t, mu, mu_next, item); });
   }
 }
 
-template <int F, int FPL>
+template <int W, int NV, int F, int LPR, int U, int MINB>
 static int run_adjoint(const AdjK& k, int launch, int grid_cap, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((k.m + 7) / 8);
+  const unsigned blocks = (unsigned)((k.m + RowSlots<LPR>::SLOTS - 1) / RowSlots<LPR>::SLOTS);
   if (launch == FLYB_LAUNCH_STEP) {
+    adj_first_kernel<W, NV, F, LPR, U, MINB><<<blocks, 256, 0, st>>>(k);
+    FLYB_CHECK_LAUNCH();
     for (int t = k.nsteps - 1; t >= 0; --t) {
-      adj_phase1_kernel<F, FPL><<<blocks, 256, 0, st>>>(k, t);
-      FLYB_CHECK_LAUNCH();
-      adj_phase2_kernel<F, FPL><<<blocks, 256, 0, st>>>(k, t);
+      adj_step_kernel<W, NV, F, LPR, U, MINB><<<blocks, 256, 0, st>>>(k, t);
       FLYB_CHECK_LAUNCH();
     }
     return 0;
@@ -189,7 +292,7 @@ static int run_adjoint(const AdjK& k, int launch, int grid_cap, cudaStream_t st)
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adj_persistent_kernel<F, FPL>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adj_persistent_kernel<W, NV, F, LPR, U, MINB>, 256, 0);
   long long grid = (long long)sms * per_sm;
   if (grid > blocks) grid = blocks;
   if (grid_cap > 0 && grid > grid_cap) grid = grid_cap;
@@ -198,27 +301,55 @@ static int run_adjoint(const AdjK& k, int launch, int grid_cap, cudaStream_t st)
   if (e != cudaSuccess) return (int)e;
   AdjK kk = k;
   void* args[] = {&kk};
-  e = cudaLaunchCooperativeKernel((void*)adj_persistent_kernel<F, FPL>, dim3((unsigned)grid), dim3(256), args, 0, st);
+  e = cudaLaunchCooperativeKernel((void*)adj_persistent_kernel<W, NV, F, LPR, U, MINB>, dim3((unsigned)grid), dim3(256), args,
+                                  0, st);
   return (int)e;
 }
 
-#define FLYB_ADJ_DISPATCH(B, CALL)                                     \
-  do {                                                                 \
-    if ((B) == 1) { constexpr int F = 1, FPL = 1; return CALL; }       \
-    if ((B) <= 2) { constexpr int F = 2, FPL = 1; return CALL; }       \
-    if ((B) <= 4) { constexpr int F = 4, FPL = 1; return CALL; }       \
-    if ((B) <= 8) { constexpr int F = 8, FPL = 1; return CALL; }       \
-    if ((B) <= 16) { constexpr int F = 16, FPL = 1; return CALL; }     \
-    if ((B) <= 32) { constexpr int F = 32, FPL = 1; return CALL; }     \
-    if ((B) <= 64) { constexpr int F = 32, FPL = 2; return CALL; }     \
-    if ((B) <= 128) { constexpr int F = 32, FPL = 4; return CALL; }    \
-    if ((B) <= 256) { constexpr int F = 32, FPL = 8; return CALL; }    \
-    return FLYB_ETOOBIG;                                               \
-  } while (0)
+// The kernel shape for a batch, by the rule of the forward substep: the widest vectors the batch and
+// the arrays allow on the fewest lanes; one or two flies leave a slot of 8 or 16 lanes per row, a
+// lobe of few rows a whole warp.
+static int run_adjoint_shape(const AdjK& k, int launch, int cap, cudaStream_t st) {
+  const void* const arrays[] = {k.lam_v, k.lam_a, k.mu0, k.mu1, k.v_hist, k.inp_hist};
+  const int B = k.batch, w = vector_width(B, arrays);
+  const bool few = k.m <= 148 * 64;
+#define FLYB_RUN(...) return run_adjoint<__VA_ARGS__>(k, launch, cap, st)
+  if (B > 256) return FLYB_ETOOBIG;
+  const int vectors = B / w;
+  if (w == 4) {
+    if (vectors == 1) { if (few) FLYB_RUN(4, 1, 1, 32, 2, 4); else FLYB_RUN(4, 1, 1, 8, 4, 4); }
+    if (vectors == 2) FLYB_RUN(4, 1, 2, 16, 4, 4);
+    if (vectors <= 4) FLYB_RUN(4, 1, 4, 32, 4, 4);
+    if (vectors <= 8) FLYB_RUN(4, 1, 8, 32, 4, 4);
+    if (vectors <= 16) FLYB_RUN(4, 1, 16, 32, 4, 4);
+    if (vectors <= 32) FLYB_RUN(4, 1, 32, 32, 4, 4);
+    FLYB_RUN(4, 2, 32, 32, 2, 3);
+  }
+  if (w == 2) {
+    if (vectors == 1) { if (few) FLYB_RUN(2, 1, 1, 32, 2, 4); else FLYB_RUN(2, 1, 1, 8, 8, 4); }
+    if (vectors == 2) FLYB_RUN(2, 1, 2, 16, 8, 4);
+    if (vectors <= 4) FLYB_RUN(2, 1, 4, 32, 4, 4);
+    if (vectors <= 8) FLYB_RUN(2, 1, 8, 32, 4, 4);
+    if (vectors <= 16) FLYB_RUN(2, 1, 16, 32, 4, 4);
+    if (vectors <= 32) FLYB_RUN(2, 1, 32, 32, 4, 4);
+    if (vectors <= 64) FLYB_RUN(2, 2, 32, 32, 4, 4);
+    FLYB_RUN(2, 4, 32, 32, 2, 3);
+  }
+  if (B == 1) { if (few) FLYB_RUN(1, 1, 1, 32, 4, 4); else FLYB_RUN(1, 1, 1, 8, 8, 4); }
+  if (B == 2) FLYB_RUN(1, 1, 2, 16, 4, 4);
+  if (B <= 4) FLYB_RUN(1, 1, 4, 32, 8, 4);
+  if (B <= 8) FLYB_RUN(1, 1, 8, 32, 8, 4);
+  if (B <= 16) FLYB_RUN(1, 1, 16, 32, 8, 4);
+  if (B <= 32) FLYB_RUN(1, 1, 32, 32, 8, 4);
+  if (B <= 64) FLYB_RUN(1, 2, 32, 32, 4, 4);
+  if (B <= 128) FLYB_RUN(1, 4, 32, 32, 4, 3);
+  FLYB_RUN(1, 8, 32, 32, 2, 3);
+#undef FLYB_RUN
+}
 
 int adjoint_blocks_per_sm() {
   int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_persistent_kernel<1, 1>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_persistent_kernel<1, 1, 1, 8, 8, 4>, 256, 0);
   return b;
 }
 
@@ -274,5 +405,5 @@ FLYB_API int flyb_optic_adjoint(const flyb_adjoint_args* a, void* stream) {
   AdjK k{a->m, a->batch, a->nsteps, a->t_ptr, a->t_col, a->t_w, a->t_perm, a->v_hist, a->inp_hist, a->a, a->b,
          a->gr, a->ga, a->aad, a->lam_v, a->lam_a, a->mu, a->lam_tmp, a->g_edge, a->g_a, a->status, a->sync};
   cudaStream_t st = (cudaStream_t)stream;
-  FLYB_ADJ_DISPATCH(a->batch, (run_adjoint<F, FPL>(k, a->launch, a->grid, st)));
+  return run_adjoint_shape(k, a->launch, a->grid, st);
 }

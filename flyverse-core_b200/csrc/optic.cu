@@ -12,7 +12,7 @@
 // of the final state is left for the next call (FLYB_OPTIC_DR_VALID).
 #include <mutex>
 
-#include "common.cuh"
+#include "flies.cuh"
 
 namespace flyb {
 
@@ -52,33 +52,6 @@ __device__ __forceinline__ void load_x(const float* __restrict__ p, float (&x)[F
 // independent ones before it consumes any (fewer when each gather is already a wide vector).
 template <int FPL>
 struct Unroll { static constexpr int U = FPL <= 2 ? 8 : (FPL == 4 ? 4 : 2); };
-
-// How the flies of a unit lie on the F fly lanes of a row slot: W consecutive flies per vector (a 4-,
-// 8- or 16-byte access, W dividing the batch), NV vectors per lane, F vectors apart. A lane's
-// vector is inside the batch as a whole or not at all.
-template <int W, int NV, int F>
-struct Flies {
-  static constexpr int FPL = W * NV;                               // flies per lane
-  static __device__ __forceinline__ int at(int f, int v) { return (f + v * F) * W; }
-};
-
-template <int W>
-__device__ __forceinline__ void load_w(const float* p, float* x) {
-  if constexpr (W == 1) {
-    x[0] = *p;
-  } else if constexpr (W == 2) {
-    const float2 q = *reinterpret_cast<const float2*>(p); x[0] = q.x; x[1] = q.y;
-  } else {
-    const float4 q = *reinterpret_cast<const float4*>(p); x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
-  }
-}
-
-template <int W>
-__device__ __forceinline__ void store_w(float* p, const float* x) {
-  if constexpr (W == 1) *p = x[0];
-  else if constexpr (W == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-  else *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-}
 
 // One {column, weight} entry. Where one load of the warp covers whole sectors of entries (4 lane
 // groups or more) the entries leave L1 to the gathered vector, much of which stays there at one
@@ -214,16 +187,10 @@ __device__ __forceinline__ void optic_row(const OpticK& k, int s, int row, bool 
   }
 }
 
-template <int LPR>
-struct OpticShape {
-  static constexpr int RPW = 32 / LPR;           // row slots per warp
-  static constexpr int SLOTS = 8 * RPW;          // row slots per 256-thread block
-};
-
 // Number of block work items of one substep: one per long row, then blocks of SLOTS short rows.
 template <int LPR>
 __host__ __device__ __forceinline__ long long optic_items(int m, int n_long) {
-  constexpr int SLOTS = OpticShape<LPR>::SLOTS;
+  constexpr int SLOTS = RowSlots<LPR>::SLOTS;
   return n_long + (m - n_long + SLOTS - 1) / SLOTS;
 }
 
@@ -234,7 +201,7 @@ __host__ __device__ __forceinline__ long long optic_items(int m, int n_long) {
 template <int W, int NV, int F, int LPR, int U>
 __device__ __forceinline__ void optic_item(const OpticK& k, int s, const float* dr_in, float* dr_out, long long item,
                                            float* red) {
-  using S = OpticShape<LPR>;
+  using S = RowSlots<LPR>;
   constexpr int FPL = W * NV;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = lane / LPR, sl = lane % LPR;
   const int gslot = warp * S::RPW + slot;
@@ -282,7 +249,7 @@ __global__ void optic_init_kernel(OpticK k) {
 // full SM of 64 warps keeps gathers in flight.
 template <int W, int NV, int F, int LPR, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) optic_step_kernel(OpticK k, int s) {
-  __shared__ float red[OpticShape<LPR>::SLOTS * F * W * NV];
+  __shared__ float red[RowSlots<LPR>::SLOTS * F * W * NV];
   const float* in = (s & 1) ? k.buf1 : k.buf0;
   float* out = (s & 1) ? k.buf0 : k.buf1;
   optic_item<W, NV, F, LPR, U>(k, s, in, out, blockIdx.x, red);
@@ -290,7 +257,7 @@ __global__ void __launch_bounds__(256, MINB) optic_step_kernel(OpticK k, int s) 
 
 template <int W, int NV, int F, int LPR, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) optic_persistent_kernel(OpticK k) {
-  __shared__ float red[OpticShape<LPR>::SLOTS * F * W * NV];
+  __shared__ float red[RowSlots<LPR>::SLOTS * F * W * NV];
   __shared__ unsigned next;
   int generation = 0;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -303,20 +270,10 @@ __global__ void __launch_bounds__(256, MINB) optic_persistent_kernel(OpticK k) {
   for (int s = 0; s < k.nsteps; ++s) {
     const float* in = (s & 1) ? k.buf1 : k.buf0;
     float* out = (s & 1) ? k.buf0 : k.buf1;
-    // Items are handed out as blocks come for them (long rows first, then shorter and shorter ones):
-    // the first gridDim.x <= items by block, the others by a count in sync[1], which grows by one per
-    // item and so by `items` per substep. Thread 0 asks for the next item beside the current one.
     // (Asking three items ahead, with the next rows' bounds on their way: 34.5 us against 32.0 at
     // one fly, 59 against 55 at 12: the gathers, not the row bounds, are what the warps wait for.)
-    for (long long item = blockIdx.x; item < items;) {
-      unsigned given = 0;
-      if (threadIdx.x == 0) given = (unsigned)atomicAdd(&k.sync[1], 1) - (unsigned)(s * items);
-      optic_item<W, NV, F, LPR, U>(k, s, in, out, item, red);
-      if (threadIdx.x == 0) next = given;
-      __syncthreads();
-      item = (long long)gridDim.x + next;
-      __syncthreads();
-    }
+    deal_items(&k.sync[1], (unsigned)s, items, &next,
+               [&](long long item) { optic_item<W, NV, F, LPR, U>(k, s, in, out, item, red); });
     if (s + 1 < k.nsteps && !grid_barrier(k.sync, k.status, generation, s)) return;
   }
 }
@@ -377,18 +334,6 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
     return FLYB_ETOOBIG;                                               \
   } while (0)
 
-// Widest vector access the batch and the arrays allow: W flies, W dividing the batch and every array
-// W floats aligned.
-static int vector_width(const OpticK& k) {
-  const void* arrays[] = {k.v, k.adapt, k.buf0, k.buf1, k.pr, k.spk, k.v_hist, k.inp_hist};
-  for (int w = 4; w > 1; w >>= 1) {
-    bool ok = k.batch % w == 0;
-    for (const void* p : arrays) ok = ok && (reinterpret_cast<uintptr_t>(p) & (4 * w - 1)) == 0;
-    if (ok) return w;
-  }
-  return 1;
-}
-
 // The substep's kernel shape for a batch, k.batch <= 256. Variant 0: vectors as wide as the batch
 // allows, spread over the fewest fly lanes, so that a warp instruction gathers for as many entries
 // as it can: the gathers then run at the L2's rate instead of the issue rate (89,390 units, 6 M
@@ -399,7 +344,8 @@ static int vector_width(const OpticK& k) {
 // other variants are what the autotuner tries beside it; one that the vector width rules out runs
 // as variant 0, an unknown one is an error.
 static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cudaStream_t st) {
-  const int B = k.batch, w = vector_width(k);
+  const void* const arrays[] = {k.v, k.adapt, k.buf0, k.buf1, k.pr, k.spk, k.v_hist, k.inp_hist};
+  const int B = k.batch, w = vector_width(B, arrays);
   const bool few = k.m <= 148 * 64;          // rows that a warp each would still hold on the SMs
 #define FLYB_RUN(...) return run_optic<__VA_ARGS__>(k, launch, cap, st)
   if (B > 256) return FLYB_ETOOBIG;
