@@ -536,11 +536,13 @@ __device__ __forceinline__ void pull_fetch(const LifK& k, const unsigned* __rest
 
 // The chunk's contribution for every step of the group: per step and fly group, the transposed
 // mask m of the inputs that spiked and base x popc(m) + sum_{q < Q} 2^q popc(m & plane_q), Q the
-// chunk's plane count as a template argument (chunk_sums dispatches on it once per chunk). Steps
-// of the group outside the pull's range are summed too (one code path, no per-step tests) and
-// never written.
-template <int G, int L, int P, int Q>
-__device__ __forceinline__ void chunk_sums_q(const Transpose32& transpose, const PullChunk<G * L, P>& x,
+// chunk's plane count as a template argument (chunk_sums dispatches on it once per chunk). A pull
+// of a whole group sums every step in one code path without tests; a pull of one or two steps
+// (PART) leaves out the steps outside its range [lo, hi): 15 M synapses, 64 flies, one step of four
+// 213 -> 148 us and two 218 -> 189 (the group: 232); with more steps the tests cost what they save
+// (32 flies, four of eight: 248 -> 259).
+template <int G, int L, int P, int Q, bool PART>
+__device__ __forceinline__ void chunk_sums_q(const Transpose32& transpose, const PullChunk<G * L, P>& x, int lo, int hi,
                                              int (&acc)[G * L]) {
   const int base = x.meta >> 5;
   unsigned pl[Q > 0 ? Q : 1];
@@ -548,6 +550,7 @@ __device__ __forceinline__ void chunk_sums_q(const Transpose32& transpose, const
   for (int q = 0; q < Q; ++q) pl[q] = P == 0 ? __ballot_sync(0xffffffffu, (x.ex >> q) & 1u) : x.pl[q];
 #pragma unroll
   for (int u = 0; u < L; ++u) {
+    if (PART && (u < lo || u >= hi)) continue;          // warp-uniform
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const unsigned m = transpose(x.w[g * L + u]);
@@ -559,11 +562,11 @@ __device__ __forceinline__ void chunk_sums_q(const Transpose32& transpose, const
   }
 }
 
-template <int G, int L, int P>
-__device__ __forceinline__ void chunk_sums(const Transpose32& transpose, const PullChunk<G * L, P>& x,
+template <int G, int L, int P, bool PART>
+__device__ __forceinline__ void chunk_sums(const Transpose32& transpose, const PullChunk<G * L, P>& x, int lo, int hi,
                                            int (&acc)[G * L]) {
   constexpr int QMAX = P == 0 ? 8 : P;   // packed entries carry 8-bit excesses
-#define FLYB_CHUNK(q) case q: chunk_sums_q<G, L, P, (q <= QMAX ? q : QMAX)>(transpose, x, acc); break;
+#define FLYB_CHUNK(q) case q: chunk_sums_q<G, L, P, (q <= QMAX ? q : QMAX), PART>(transpose, x, lo, hi, acc); break;
   switch (x.meta & 31) {              // warp-uniform: one dispatch per chunk
     FLYB_CHUNK(0) FLYB_CHUNK(1) FLYB_CHUNK(2) FLYB_CHUNK(3) FLYB_CHUNK(4) FLYB_CHUNK(5) FLYB_CHUNK(6)
     FLYB_CHUNK(7) FLYB_CHUNK(8)
@@ -588,7 +591,7 @@ __device__ __forceinline__ void chunk_sums(const Transpose32& transpose, const P
 // row's first chunk), and are stored when it ends: the slots end with the same integers an add
 // into them would leave, without a load waiting at the end of each row. Rows without inputs are
 // not touched.
-template <int G, int L, int P>
+template <int G, int L, int P, bool PART>
 __device__ __forceinline__ void pull_pass(const LifK& k, const unsigned* __restrict__ bits, int r0, int r1, int lo,
                                           int hi, int ws0, int lane) {
   constexpr int NW = G * L;
@@ -636,7 +639,7 @@ __device__ __forceinline__ void pull_pass(const LifK& k, const unsigned* __restr
       end_row();
       start_row();
     }
-    chunk_sums<G, L, P>(transpose, cur, acc);
+    chunk_sums<G, L, P, PART>(transpose, cur, lo, hi, acc);
     cur = nxt;
     pre_next = pre_after;
   }
@@ -658,7 +661,7 @@ __device__ __forceinline__ void pull_pass(const LifK& k, const unsigned* __restr
 // the warp's row block are counted from the same words. The last block to finish moves pull_state
 // on by nsteps (every block has read it by then).
 constexpr int kPullBlock = 256, kPullBlocksPerSm = 3;   // launch shape of the pull kernel
-template <int G, int L, int P>
+template <int G, int L, int P, bool PART>
 __global__ void __launch_bounds__(kPullBlock, kPullBlocksPerSm) lif_pull_kernel(LifK k, int nsteps) {
   constexpr int NW = G * L;
   const long long done = k.pull_state[0];
@@ -678,7 +681,7 @@ __global__ void __launch_bounds__(kPullBlock, kPullBlocksPerSm) lif_pull_kernel(
     // write slot of step grp * L + u: D slots after its read slot (consecutive steps, consecutive slots)
     const int ws0 = pos_mod(rp_done + (grp * L - done) + k.n_delay, k.R);
     if (r0 >= r1) continue;
-    pull_pass<G, L, P>(k, bits, r0, r1, lo, hi, ws0, lane);
+    pull_pass<G, L, P, PART>(k, bits, r0, r1, lo, hi, ws0, lane);
     if (k.events) {                          // events of presynaptic neurons r0 .. r1 in these steps
       for (int j = r0 + lane; j < r1; j += 32) {
         unsigned wj[NW];
@@ -713,22 +716,26 @@ __global__ void __launch_bounds__(kPullBlock, kPullBlocksPerSm) lif_pull_kernel(
 
 // The pull kernel uses no shared memory: it asks for the largest L1, where part of the spike words
 // its gathers read stays resident, and runs as one wave of resident blocks.
-template <int G, int L, int P>
+template <int G, int L, int P, bool PART>
 static void launch_pull_glp(const LifK& k, int nsteps, int sms, cudaStream_t st) {
   static int per_sm = 0;                 // resident blocks: one wave, each warp a longer row stream
   if (!per_sm) {
-    cudaFuncSetAttribute(lif_pull_kernel<G, L, P>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lif_pull_kernel<G, L, P>, kPullBlock, 0);
+    cudaFuncSetAttribute(lif_pull_kernel<G, L, P, PART>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lif_pull_kernel<G, L, P, PART>, kPullBlock, 0);
     if (per_sm < 1) per_sm = 1;
   }
   const int grid = k.pull_grid > 0 && k.pull_grid < sms * per_sm ? k.pull_grid : sms * per_sm;
-  lif_pull_kernel<G, L, P><<<grid, kPullBlock, 0, st>>>(k, nsteps);
+  lif_pull_kernel<G, L, P, PART><<<grid, kPullBlock, 0, st>>>(k, nsteps);
 }
 
 template <int G, int L>
 static void launch_pull_gl(const LifK& k, int nsteps, int sms, cudaStream_t st) {
-  if (k.pull_nplanes == 0) launch_pull_glp<G, L, 0>(k, nsteps, sms, st);
-  else launch_pull_glp<G, L, 16>(k, nsteps, sms, st);
+  if constexpr (L > 1)
+    if (nsteps < L && nsteps <= 2)
+      return k.pull_nplanes == 0 ? launch_pull_glp<G, L, 0, true>(k, nsteps, sms, st)
+                                 : launch_pull_glp<G, L, 16, true>(k, nsteps, sms, st);
+  if (k.pull_nplanes == 0) launch_pull_glp<G, L, 0, false>(k, nsteps, sms, st);
+  else launch_pull_glp<G, L, 16, false>(k, nsteps, sms, st);
 }
 
 // Steps per group a batch width allows: 8 / G (one sector per input and group), or 1.

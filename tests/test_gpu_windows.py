@@ -105,3 +105,25 @@ def test_brain_by_windows_equals_one_step_per_call(batch, launch, pull, std_u):
         assert a.synaptic_events == b.synaptic_events
     assert float(a.spike_counts.sum()) > 0
     a.check()
+
+
+@pytest.mark.parametrize("batch", [32, 64, 128])
+@pytest.mark.parametrize("counts", [1, 300])            # packed entries, and counts that need the plane table
+def test_pulls_of_parts_of_groups_equal_the_scatter(batch, counts):
+    """Calls of 1, 2, 3, ... steps, which pull parts of groups and across group ends, against the scatter."""
+    cfg = synthetic.lif_config1(seed=2, n=1500, edges=30_000)
+    cfg.c.W.data[::7] *= counts
+    both = []
+    for pull in (False, True):
+        b = Brain(cfg.c, LIFParams(**cfg.params), device="cuda", seed=9, batch=batch, launch="step")
+        b.record_activity, b.pull = True, pull
+        b.set_poisson(cfg.poisson_idx, 400.0)
+        b.set_drive(np.arange(cfg.c.n), 6.9)
+        b._make_args()
+        for steps in (1, 1, 2, 3, 1, 2, 2, 5, 1, 6, 20):
+            b.step(steps)
+        b.check()
+        both.append(b)
+    a, b = both
+    assert b._pull_active() and b._pull_planes_n == (0 if counts == 1 else 16) and float(a.spike_counts.sum()) > 0
+    assert torch.equal(a.ring, b.ring) and torch.equal(a.v, b.v) and a.synaptic_events == b.synaptic_events
