@@ -137,8 +137,12 @@ def launch_trace(scene: torch.Tensor, shape: tuple, detail: float, out: torch.Te
                        shared_origin=int(shared_origin), samples=1 if weights is None else weights.numel(),
                        detail=float(detail), scene=_abi.ptr(scene), origins=_abi.ptr(origins), dirs=_abi.ptr(dirs),
                        eye_dirs=_abi.ptr(eye_dirs), pose=_abi.ptr(pose), weights=_abi.ptr(weights), out=_abi.ptr(out))
-    with torch.cuda.device(out.device):
-        rc = _abi.lib().flyb_trace(ct.byref(a), torch.cuda.current_stream(out.device).cuda_stream)
+    stream = torch.cuda.current_stream(out.device).cuda_stream
+    if torch.cuda.current_device() == out.device.index:
+        rc = _abi.lib().flyb_trace(ct.byref(a), stream)
+    else:
+        with torch.cuda.device(out.device):
+            rc = _abi.lib().flyb_trace(ct.byref(a), stream)
     if rc:
         raise RuntimeError(f"flyb_trace: error {rc}")
 
