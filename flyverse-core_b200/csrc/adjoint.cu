@@ -18,9 +18,10 @@
 // writer. With lam of step t - 1 in hand the slot goes on to mu_{t-1} and the g_a term of its
 // unit, so a reverse step is one pass over the rows and, mu being double-buffered, one grid
 // barrier. Bound: the entries with their accumulator (16 bytes per edge and step) and the gathers of
-// mu, both out of L2. Measured per reverse step: 89,390 units, 6 M entries, one fly 63 -> 52 us; 20,000
-// units, 1.34 M entries, 16 flies 85 -> 25 us (four lanes of four flies instead of sixteen of one;
-// the per-edge sums by halving exchanges).
+// mu, both out of L2. Measured per reverse step: 89,390 units, 6 M entries, one fly 67 -> 45 us, four
+// flies 149 -> 48 us; 20,000 units, 1.34 M entries, 16 flies 85 -> 25 us (four lanes of four flies
+// instead of sixteen of one; the per-edge sums by halving exchanges; the accumulators requested
+// beside the gathers).
 #include "flies.cuh"
 
 namespace flyb {
@@ -66,14 +67,27 @@ __device__ __forceinline__ void adj_unit(const AdjK& k, int t, int j, bool on, i
   if (on && sl == 0) k.g_a[j] = k.g_a[j] + part;
 }
 
-// Sums ge[u], u < U, over the F fly lanes of the group and adds them to the accumulators of the
-// entries base + u * stride. While two or more entries are left a halving exchange leaves each
-// half of the lanes with half of the entries (U = 4, F = 16: 5 exchanges instead of 16); the
-// remaining exchanges sum whole.
+// The edges whose accumulators a lane writes after the sums of U entries over F fly lanes (add_edges):
+// COUNT of them from entry `first` on, by one lane in SAME.
 template <int F, int U>
-__device__ __forceinline__ void add_edges(const AdjK& k, float (&ge)[U], int base, int stride, int e1, int f) {
-  int first = 0;
-  int left = U;
+struct EdgeOwner {
+  static constexpr int COUNT = U > F ? U / F : 1, SAME = F > U ? F / U : 1;
+  static __device__ __forceinline__ int first(int f) {
+    int first = 0;
+#pragma unroll
+    for (int o = F / 2, n = U; o >= 1 && n > 1; o >>= 1) {
+      n >>= 1;
+      first += f & o ? n : 0;
+    }
+    return first;
+  }
+};
+
+// Sums ge[u], u < U, over the F fly lanes of the group; lane f is left with the sums of the entries it
+// owns. While two or more entries are left a halving exchange leaves each half of the lanes with
+// half of the entries (U = 4, F = 16: 5 exchanges instead of 16); the remaining ones sum whole.
+template <int F, int U>
+__device__ __forceinline__ void sum_edges(float (&ge)[U], int f) {
 #pragma unroll
   for (int o = F / 2, n = U; o >= 1; o >>= 1) {
     if (n > 1) {
@@ -85,21 +99,8 @@ __device__ __forceinline__ void add_edges(const AdjK& k, float (&ge)[U], int bas
           const float send = up ? ge[q] : ge[q + n], keep = up ? ge[q + n] : ge[q];
           ge[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
-      first += up ? n : 0;
-      left = n;
     } else {
       ge[0] = ge[0] + __shfl_xor_sync(0xffffffffu, ge[0], o);
-    }
-  }
-  // lanes that hold the same sums: the one whose remaining lane bits are zero writes
-  constexpr int SAME = F > U ? F / U : 1;
-  if (f & (SAME - 1)) return;
-#pragma unroll
-  for (int q = 0; q < U; ++q) {
-    const int e = base + (first + q) * stride;
-    if (q < left && e < e1) {
-      const int pe = k.t_perm ? k.t_perm[e] : e;
-      k.g_edge[pe] = k.g_edge[pe] + ge[q];
     }
   }
 }
@@ -121,6 +122,9 @@ __device__ __forceinline__ void adj_entries(const AdjK& k, const float* mu, int 
   }
 #pragma unroll
   for (int q = 0; q < FPL; ++q) acc[q] = 0.0f;
+  using Own = EdgeOwner<F, U>;
+  const int own = Own::first(f);
+  const bool owns = (f & (Own::SAME - 1)) == 0;
   // every lane of the warp takes part in the exchanges: the slots go on to the longest one's end
   const int trips = __reduce_max_sync(0xffffffffu, (e1 - e0 + G * U - 1) / (G * U));
   for (int trip = 0, base = e0 + g; trip < trips; ++trip, base += G * U) {
@@ -132,6 +136,15 @@ __device__ __forceinline__ void adj_entries(const AdjK& k, const float* mu, int 
       const bool ok = e < e1;
       ii[u] = ok ? __ldg(&k.t_col[e]) : 0;
       ww[u] = ok ? __ldg(&k.t_w[e]) : 0.0f;
+    }
+    // the accumulators this lane will add to, on their way beside the gathers
+    int at[Own::COUNT];
+    float old[Own::COUNT];
+#pragma unroll
+    for (int q = 0; q < Own::COUNT; ++q) {
+      const int e = base + (own + q) * G;
+      at[q] = owns && e < e1 ? (k.t_perm ? k.t_perm[e] : e) : -1;
+      old[q] = at[q] >= 0 ? k.g_edge[at[q]] : 0.0f;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -150,7 +163,10 @@ __device__ __forceinline__ void adj_entries(const AdjK& k, const float* mu, int 
           ge[u] = fmaf(m, dr[q], ge[u]);
         }
     }
-    add_edges<F, U>(k, ge, base, G, e1, f);
+    sum_edges<F, U>(ge, f);
+#pragma unroll
+    for (int q = 0; q < Own::COUNT; ++q)
+      if (at[q] >= 0) k.g_edge[at[q]] = old[q] + ge[q];
   }
 #pragma unroll
   for (int o = F; o < LPR; o <<= 1)
@@ -326,8 +342,8 @@ static int run_adjoint_shape(const AdjK& k, int launch, int cap, cudaStream_t st
     FLYB_RUN(4, 2, 32, 32, 2, 3);
   }
   if (w == 2) {
-    if (vectors == 1) { if (few) FLYB_RUN(2, 1, 1, 32, 2, 4); else FLYB_RUN(2, 1, 1, 8, 8, 4); }
-    if (vectors == 2) FLYB_RUN(2, 1, 2, 16, 8, 4);
+    if (vectors == 1) { if (few) FLYB_RUN(2, 1, 1, 32, 2, 4); else FLYB_RUN(2, 1, 1, 8, 4, 4); }
+    if (vectors == 2) FLYB_RUN(2, 1, 2, 16, 4, 4);
     if (vectors <= 4) FLYB_RUN(2, 1, 4, 32, 4, 4);
     if (vectors <= 8) FLYB_RUN(2, 1, 8, 32, 4, 4);
     if (vectors <= 16) FLYB_RUN(2, 1, 16, 32, 4, 4);
@@ -335,7 +351,7 @@ static int run_adjoint_shape(const AdjK& k, int launch, int cap, cudaStream_t st
     if (vectors <= 64) FLYB_RUN(2, 2, 32, 32, 4, 4);
     FLYB_RUN(2, 4, 32, 32, 2, 3);
   }
-  if (B == 1) { if (few) FLYB_RUN(1, 1, 1, 32, 4, 4); else FLYB_RUN(1, 1, 1, 8, 8, 4); }
+  if (B == 1) { if (few) FLYB_RUN(1, 1, 1, 32, 4, 4); else FLYB_RUN(1, 1, 1, 8, 8, 3); }
   if (B == 2) FLYB_RUN(1, 1, 2, 16, 4, 4);
   if (B <= 4) FLYB_RUN(1, 1, 4, 32, 8, 4);
   if (B <= 8) FLYB_RUN(1, 1, 8, 32, 8, 4);
@@ -349,7 +365,7 @@ static int run_adjoint_shape(const AdjK& k, int launch, int cap, cudaStream_t st
 
 int adjoint_blocks_per_sm() {
   int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_persistent_kernel<1, 1, 1, 8, 8, 4>, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, adj_persistent_kernel<1, 1, 1, 8, 8, 3>, 256, 0);
   return b;
 }
 

@@ -164,14 +164,17 @@ def spmm(M: DeviceCSR, x: torch.Tensor, y: torch.Tensor, *, x_index=None, x_div=
         raise RuntimeError(f"flyb_spmm: error {rc}")
 
 
-def long_row_entries(nnz: int, sms: int = 148) -> int:
-    """Entries above which a row is split across a whole block (OpticCore.set_long_rows): three times
-    the entries that each of the ~48 resident warps per SM has to itself, between 96 and 512. A large
-    lobe has work enough that only the longest rows hold it up, and splitting costs a block's
-    reduction; in a small one a warp's single row may last as long as the whole substep. Measured
-    per substep at thresholds 192 / 512: 6 M entries 44.9 / 34.8 us at one fly and 121 / 115 at 64;
-    at 96 / 192: 0.1 M entries 8.5 / 12.6 us at 64 flies."""
-    return max(96, min(512, 3 * nnz // (48 * sms)))
+def long_row_entries(nnz: int, batch: int) -> int:
+    """Entries above which a row is split across a whole block (OpticCore.set_long_rows): as many as one
+    row slot gets through in a third of the substep, between 192 (96 from 16 flies on) and 512. A slot
+    takes ~64 entries per pass of ~0.8 us at a few flies, 512 / batch at more; a substep lasts about
+    30 + 1.4 x batch us at 6 M entries. Splitting costs a block's reduction, so a large lobe splits
+    its longest rows only; in a small one a single slot's row could outlast everything else. Measured
+    per substep at thresholds 192 / 512: 6 M entries 44.9 / 34.8 us at one fly, 121 / 115 at 64;
+    1.3 M entries 15.8 / 18.9 at 4; at 96 / 192: 0.1 M entries 8.5 / 12.6 us at 64 flies, 4.6 / 4.2 at one."""
+    substep_us = nnz / 6e6 * (30.0 + 1.4 * batch)
+    per_pass = min(64.0, 512.0 / batch)
+    return int(max(192 if batch < 16 else 96, min(512, per_pass * substep_us / (3 * 0.8))))
 
 
 class OpticCore:
@@ -205,7 +208,7 @@ class OpticCore:
         self.launch = launch
         self.variant = 0                 # kernel shape (flyb_optic_args.variant), set by the autotuner
         self.grid = 0                    # persistent launches: block cap (0 = every resident block)
-        self.set_long_rows(long_row_entries(self.W.nnz, _sm_count(self.device)))
+        self.set_long_rows(long_row_entries(self.W.nnz, self.B))
         M, B, dev = self.m, self.B, self.device
         self.v_s = torch.zeros(M, B, device=dev)
         self.adapt_s = torch.zeros(M, B, device=dev)

@@ -58,5 +58,6 @@ def test_unaligned_state_matches_oracle(batch, offset):
     check(1200, batch, offset=offset)
 
 
-def test_long_row_threshold_follows_the_entries_per_warp():
-    assert [long_row_entries(n) for n in (0, 100_000, 500_000, 6_000_000)] == [96, 96, 211, 512]
+def test_long_row_threshold_follows_the_lobe_and_the_batch():
+    cases = {(0, 1): 192, (100_000, 64): 96, (1_340_000, 4): 212, (6_000_000, 1): 512, (6_000_000, 12): 512}
+    assert {k: long_row_entries(*k) for k in cases} == cases
