@@ -339,7 +339,8 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
 // as it can: the gathers then run at the L2's rate instead of the issue rate (89,390 units, 6 M
 // entries, one substep: 12 flies 162 us with 16 lanes of one fly, 55 us with 4 lanes of four; 24
 // flies 294 -> 80; 64 flies 254 -> 115 us and 128 flies 416 -> 254 us with the registers bounded for
-// six and four blocks per SM). Narrow rows leave lanes over for entries; a
+// six and four blocks per SM). Rows above 75,776 give a row of 4 or 8 fly lanes half a warp (12 flies,
+// 89,390 units 59 -> 50 us; 50,000 units 32.5 -> 34.3, so not below). Narrow rows leave lanes over for entries; a
 // lobe of few rows gives each row a whole warp (LPR 32), so that its rows still fill the SMs. The
 // other variants are what the autotuner tries beside it; one that the vector width rules out runs
 // as variant 0, an unknown one is an error.
@@ -347,6 +348,7 @@ static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cu
   const void* const arrays[] = {k.v, k.adapt, k.buf0, k.buf1, k.pr, k.spk, k.v_hist, k.inp_hist};
   const int B = k.batch, w = vector_width(B, arrays);
   const bool few = k.m <= 148 * 64;          // rows that a warp each would still hold on the SMs
+  const bool many = k.m > 148 * 512;         // rows enough to halve their lanes without idling any
 #define FLYB_RUN(...) return run_optic<__VA_ARGS__>(k, launch, cap, st)
   if (B > 256) return FLYB_ETOOBIG;
   if (variant < 0 || variant > 5) return FLYB_EINVAL;
@@ -382,9 +384,9 @@ static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cu
   const int vectors = B / w;
   if (w == 4) {
     if (vectors == 1) { if (few) FLYB_RUN(4, 1, 1, 32, 2, 4); else FLYB_RUN(4, 1, 1, 8, 4, 4); }
-    if (vectors == 2) { if (few) FLYB_RUN(4, 1, 2, 32, 4, 4); else FLYB_RUN(4, 1, 2, 16, 4, 4); }
-    if (vectors <= 4) FLYB_RUN(4, 1, 4, 32, 4, 5);
-    if (vectors <= 8) FLYB_RUN(4, 1, 8, 32, 4, 5);
+    if (vectors == 2) { if (few) FLYB_RUN(4, 1, 2, 32, 4, 4); else if (many) FLYB_RUN(4, 1, 2, 16, 4, 6); else FLYB_RUN(4, 1, 2, 16, 4, 4); }
+    if (vectors <= 4) { if (many) FLYB_RUN(4, 1, 4, 16, 4, 5); else FLYB_RUN(4, 1, 4, 32, 4, 5); }
+    if (vectors <= 8) { if (many) FLYB_RUN(4, 1, 8, 32, 4, 6); else FLYB_RUN(4, 1, 8, 32, 4, 5); }
     if (vectors <= 16) FLYB_RUN(4, 1, 16, 32, 4, 6);
     if (vectors <= 32) FLYB_RUN(4, 1, 32, 32, 4, 4);
     FLYB_RUN(4, 2, 32, 32, 2, 4);
@@ -392,7 +394,7 @@ static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cu
   if (w == 2) {
     if (vectors == 1) { if (few) FLYB_RUN(2, 1, 1, 32, 4, 4); else FLYB_RUN(2, 1, 1, 8, 8, 4); }
     if (vectors == 2) FLYB_RUN(2, 1, 2, 16, 8, 4);
-    if (vectors <= 4) FLYB_RUN(2, 1, 4, 32, 4, 5);
+    if (vectors <= 4) { if (many) FLYB_RUN(2, 1, 4, 16, 4, 5); else FLYB_RUN(2, 1, 4, 32, 4, 5); }
     if (vectors <= 8) FLYB_RUN(2, 1, 8, 32, 8, 4);
     if (vectors <= 16) FLYB_RUN(2, 1, 16, 32, 8, 4);
     if (vectors <= 32) FLYB_RUN(2, 1, 32, 32, 8, 4);
@@ -400,8 +402,8 @@ static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cu
     FLYB_RUN(2, 4, 32, 32, 2, 4);
   }
   if (B == 2) FLYB_RUN(1, 1, 2, 16, 8, 4);
-  if (B <= 4) FLYB_RUN(1, 1, 4, 32, 8, 4);
-  if (B <= 8) FLYB_RUN(1, 1, 8, 32, 8, 4);
+  if (B <= 4) { if (many) FLYB_RUN(1, 1, 4, 16, 8, 4); else FLYB_RUN(1, 1, 4, 32, 8, 4); }
+  if (B <= 8) { if (many) FLYB_RUN(1, 1, 8, 16, 8, 4); else FLYB_RUN(1, 1, 8, 32, 8, 4); }
   if (B <= 16) FLYB_RUN(1, 1, 16, 32, 8, 4);
   if (B <= 32) FLYB_RUN(1, 1, 32, 32, 8, 4);
   if (B <= 64) FLYB_RUN(1, 2, 32, 32, 4, 5);

@@ -64,6 +64,7 @@ class WholeFly:
         aad = float(np.exp(-dt_ms / o.adapt_tau_ms))
         self.optic = OpticCore(o.W_rr(), a, o.b, batch=self.B, device=self.device, gain_rr=o.gain_rr,
                                adapt_gain=o.adapt_gain, aad=aad, launch="step")
+        self.optic.single_steps = True
         dev = self.device
         # the coupling blocks keep only their non-empty rows (+ the row map): the other rows of spk_in
         # and of the drive are never written and stay zero
