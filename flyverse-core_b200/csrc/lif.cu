@@ -10,6 +10,9 @@
 // Both sums are independent of the order in which red.global.add lands, so rasters and state are
 // deterministic and equal to the C restatement in oracle/flyoracle.c bit for bit.
 //
+// Runs of more than one step go by delay windows (lif_window.cuh); the per-step kernels here run
+// single steps, neuron ranges, episode counters and runs without a raster.
+//
 // Layout: state [n][batch] (fly-minor), ring [R][n][batch]; work item t = i * batch + b.
 #include <type_traits>
 

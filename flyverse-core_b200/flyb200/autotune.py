@@ -1,9 +1,9 @@
 """Launch-parameter autotuner for the native steps, cached per (graph, batch, activity bucket).
 
-The best launch shape depends on the graph, the batch and how many cells spike per step: at B = 1
-the step is latency-bound and a persistent cooperative launch (one launch for many steps, a grid
-barrier per step) wins; at B = 64 the state streams from HBM and one launch per step, with the
-state staged through shared memory by bulk copies, keeps more bytes in flight. `tune_lif` times
+The best launch shape depends on the graph, the batch and how many cells spike per step. Calls of
+many steps go by delay windows: one cooperative launch or two launches per window, the spikes
+scattered or pulled. Engines that step by single launches stream the state from HBM every step:
+there the register and the bulk-copy kernels, block sizes and deliveries differ. `tune_lif` times
 each candidate (launch mode x block size x items per thread x spike delivery) for a few steps on a
 copy of the live state, restores the state, installs the fastest and caches it under the key;
 `tune_optic` does the same for the optic substep's launch mode and kernel shape.
