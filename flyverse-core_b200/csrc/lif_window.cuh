@@ -16,7 +16,7 @@
 // instead of one per step. The update is then bound by instruction issue (many flies) or by the
 // latency of its 18 dependent steps (one fly: ~250 cycles each), the delivery by L2 atomics (or
 // the pull's own bound). Measured on 71,618 neurons and 15 M synapses at dense firing: one fly
-// 38.7 -> 3.4 us per step; 64 flies, the update alone 55 -> 18 us per step in windows of 8; 2,000
+// 38.7 -> 3.4 us per step; 64 flies, the update alone 55 -> 17 us per step in windows of 8; 2,000
 // neurons, one fly: 5.4 -> 0.56 us per step.
 #pragma once
 
@@ -24,7 +24,11 @@ namespace flyb {
 
 constexpr int kWindowBlock = 256;
 constexpr int kWindowMax = 32;      // steps per window: lane j of a warp keeps the spike word of step j
-constexpr int kWindowAhead = 6;     // ring values loaded ahead of their steps: ~100 cycles a step against an L2 round trip
+// Ring values loaded ahead of their steps. A persistent run of few items waits for each of them (6: one
+// fly, 2,000 neurons 55.9 us per 100 steps against 57.1 with 4); the update of many items has other
+// warps to run and takes 4, with registers bounded for six blocks per SM (64 flies, 71,618 neurons,
+// 40 steps: 3040 -> 2918 us).
+constexpr int kAheadFew = 6, kAheadMany = 4;
 constexpr int kWindowBits = 4;      // spikes a thread hands over per delivery round
 constexpr int kWindowEdges = 4;     // edges a lane of the delivery keeps in flight
 
@@ -87,7 +91,7 @@ __device__ __forceinline__ float spike_value(const LifK& k, const Clk& clk, int 
 // step j until the end, where one store writes the words of all steps. Under depression the
 // spikes array keeps the resource at the window's start until the delivery has used it
 // (window_finish puts the spikes back).
-template <bool FIXED, bool STD>
+template <bool FIXED, bool STD, int AHEAD>
 __device__ __forceinline__ void window_update(const LifK& k, const Clk& clk, int s0, int K, long long base, int span) {
   using RingT = typename std::conditional<FIXED, long long, int>::type;
   const long long t = base + threadIdx.x;
@@ -134,10 +138,10 @@ __device__ __forceinline__ void window_update(const LifK& k, const Clk& clk, int
     }
   }
   const float res0 = rr;
-  // ring values in flight: the value of step j + kWindowAhead is requested when step j has used its
+  // ring values in flight: the value of step j + AHEAD is requested when step j has used its
   // own. Requests beyond the window, and those of lanes without an item, read a word nobody uses:
   // the loop then has no branch around a load.
-  RingT due[kWindowAhead];
+  RingT due[AHEAD];
   int rs = first_slot, cs = first_slot;                        // slots of the next load and of the step being run
   const RingT* from = (const RingT*)k.ring + (ok ? t : (long long)k.t_end - 1);
   const auto next_value = [&]() {
@@ -148,11 +152,11 @@ __device__ __forceinline__ void window_update(const LifK& k, const Clk& clk, int
   float spike = 0.0f;
   unsigned my_word = 0;
 #pragma unroll
-  for (int u = 0; u < kWindowAhead; ++u) due[u] = next_value();
+  for (int u = 0; u < AHEAD; ++u) due[u] = next_value();
   const unsigned forced = poisson_steps(k, clk, s0, K, t, i, b, pp);
-  for (int j0 = 0; j0 < K; j0 += kWindowAhead) {
+  for (int j0 = 0; j0 < K; j0 += AHEAD) {
 #pragma unroll
-    for (int u = 0; u < kWindowAhead; ++u) {
+    for (int u = 0; u < AHEAD; ++u) {
       const int j = j0 + u;
       if (j >= K) break;
       const RingT c = ok ? due[u] : 0;
@@ -354,8 +358,8 @@ __device__ __forceinline__ void window_finish(const LifK& k, const Clk& clk, lon
 
 // Per-step launches: one update and one delivery launch per window.
 template <bool FIXED, bool STD>
-__global__ void __launch_bounds__(kWindowBlock, FIXED ? 3 : 4) lif_window_update_kernel(LifK k, int s0, int K) {
-  window_update<FIXED, STD>(k, read_clock(k), s0, K, k.t_begin + (long long)blockIdx.x * kWindowBlock, kWindowBlock);
+__global__ void __launch_bounds__(kWindowBlock, FIXED ? 4 : 6) lif_window_update_kernel(LifK k, int s0, int K) {
+  window_update<FIXED, STD, kAheadMany>(k, read_clock(k), s0, K, k.t_begin + (long long)blockIdx.x * kWindowBlock, kWindowBlock);
 }
 
 template <bool FIXED>
@@ -378,7 +382,7 @@ __global__ void __launch_bounds__(kWindowBlock, FIXED ? 3 : 4) lif_window_persis
     const int K = kmax < k.nsteps - s0 ? kmax : k.nsteps - s0;
     const bool last = s0 + K == k.nsteps;
     for (long long base = k.t_begin + (long long)blockIdx.x * span; base < k.t_end; base += (long long)gridDim.x * span)
-      window_update<FIXED, STD>(k, clk, s0, K, base, span);
+      window_update<FIXED, STD, kAheadFew>(k, clk, s0, K, base, span);
     if (!grid_barrier(k.sync, k.status, generation, s0)) return;
     if (last && blockIdx.x == 0 && !(k.flags & FLYB_LIF_NO_ADVANCE)) advance_clock(k, clk);   // all have read it
     window_deliver<FIXED>(k, clk, s0, K, parts, sm);
