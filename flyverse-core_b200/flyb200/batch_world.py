@@ -87,6 +87,9 @@ class BatchWorld(World):
         self._pose_block = torch.zeros(self.B * 84, dtype=torch.uint8, device=device)
         self._pose = self._pose_block[:self.B * 72].view(torch.float64).view(self.B, 9)
         self._eye_pos = self._pose_block[self.B * 72:].view(torch.float32).view(self.B, 3)
+        self._pose_copied = torch.cuda.Event()     # the last poses' copy, and the stream it is on
+        self._pose_stream = None
+        self._pose_captured = False                # a captured trace reads the poses wherever it is replayed
 
     def set_pose(self, eye, forward, left, up) -> None:
         """Eye positions (B, 3) and orientations forward/left/up (B, 3 each) for the next eye
@@ -94,13 +97,20 @@ class BatchWorld(World):
         reads; the copy is complete on return, so a graph may read it from any stream."""
         self._queue_pose(eye, forward, left, up)
         torch.cuda.current_stream(self.device).synchronize()
+        self._pose_stream = None
+
+    def _capturing(self) -> bool:
+        if torch.cuda.current_device() == self.device.index:
+            return torch.cuda.is_current_stream_capturing()
+        with torch.cuda.device(self.device):
+            return torch.cuda.is_current_stream_capturing()
 
     def _queue_pose(self, eye, forward, left, up) -> None:
         """The poses' copy queued on the current stream: one block, staged in pinned memory (the
         allocator keeps it until the copy has run)."""
         if self._eye is None:
             raise ValueError("set_eye() first")
-        if torch.cuda.is_current_stream_capturing():
+        if self._capturing():
             raise RuntimeError("poses are copied from the host: set them outside the capture")
         staged = torch.empty(self.B * 84, dtype=torch.uint8, pin_memory=True)
         host = staged.numpy()
@@ -109,13 +119,24 @@ class BatchWorld(World):
             pose[:, 3 * q:3 * q + 3] = np.asarray(v, dtype=np.float64).reshape(self.B, 3)
         host[self.B * 72:].view(np.float32).reshape(self.B, 3)[:] = np.asarray(eye, dtype=np.float32).reshape(self.B, 3)
         self._pose_block.copy_(staged, non_blocking=True)
+        self._pose_stream = torch.cuda.current_stream(self.device)
+        self._pose_copied.record(self._pose_stream)
 
     @torch.no_grad()
     def trace_eye(self, out: torch.Tensor | None = None) -> torch.Tensor:
-        """(B, n_col, 4) radiance per column at the poses last given to `set_pose`: one launch,
-        capturable in a CUDA graph."""
+        """(B, n_col, 4) radiance per column at the poses last given to `set_pose` or
+        `column_radiance`: one launch, capturable in a CUDA graph."""
         if self._eye is None:
             raise ValueError("set_eye() first")
+        if self._capturing():
+            self._pose_captured = True
+        elif self._pose_stream is not None:
+            stream = torch.cuda.current_stream(self.device)
+            if stream != self._pose_stream:        # the poses were queued on another stream
+                stream.wait_event(self._pose_copied)
+        return self._trace_eye(out)
+
+    def _trace_eye(self, out: torch.Tensor | None) -> torch.Tensor:
         device = self._ready()
         eye_dirs, w, n_col = self._eye
         if out is None:
@@ -132,6 +153,10 @@ class BatchWorld(World):
         fly's scene, weighted and summed over each column's samples in sample order
         (batch_sim.py:192-201). Writes into `out` when given (e.g. FlyBrain's held radiance)."""
         # the trace follows on the same stream: nothing waits for the copy (two synchronising copies a
-        # frame kept the host from queueing the next: 64 eyes 146 -> 79 us per frame, one 63 -> 50)
-        self._queue_pose(eye, forward, left, up)
-        return self.trace_eye(out)
+        # frame kept the host from queueing the next: 64 eyes 146 -> 77 us per frame, one 63 -> 39),
+        # unless a captured trace, which may be replayed on any stream, reads the same poses
+        if self._pose_captured:
+            self.set_pose(eye, forward, left, up)
+        else:
+            self._queue_pose(eye, forward, left, up)
+        return self._trace_eye(out)
