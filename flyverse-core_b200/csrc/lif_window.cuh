@@ -121,9 +121,11 @@ __device__ __forceinline__ void window_update(const LifK& k, const Clk& clk, int
     act = k.active[i];
   }
   if (k.flags & FLYB_LIF_SKIP_FROZEN) {
-    // a warp of frozen cells at rest without input in the window: nothing changes (neural.cu:24-26)
+    // a warp of frozen cells at rest without input in the window: nothing changes (neural.cu:24-26).
+    // A cell that passes the other tests has not spiked in this run, so its spike value is looked at
+    // in the first window only: under depression the array then holds the resource.
     bool rest = act == 0.0f && pp == 0.0f && vv == P.v_rest && gg == 0.0f && dv == 0.0f && ad == 0.0f &&
-                ref == 0.0f && rt == 0.0f && (!ok || (k.spikes[t] == 0.0f && k.res[t] == 1.0f));
+                ref == 0.0f && rt == 0.0f && (!ok || ((s0 > 0 || k.spikes[t] == 0.0f) && k.res[t] == 1.0f));
     if (__all_sync(0xffffffffu, rest)) {
       int slot_of = first_slot;
       for (int j = 0; j < K; ++j) {
