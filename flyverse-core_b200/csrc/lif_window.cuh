@@ -29,7 +29,11 @@ constexpr int kWindowMax = 32;      // steps per window: lane j of a warp keeps 
 // warps to run and takes 4, with registers bounded for six blocks per SM (64 flies, 71,618 neurons,
 // 40 steps: 3040 -> 2918 us).
 constexpr int kAheadFew = 6, kAheadMany = 4;
-constexpr int kWindowBits = 4;      // spikes a thread hands over per delivery round
+constexpr int kWindowSpikes = 4;    // spikes a thread hands over per delivery round
+// Blocks per SM of a delivery launch. At dense firing the atomics of more blocks spread over more of the
+// ring than the L2 holds (70,000 neurons, 256 flies in step, 20 steps at a delay of 6: 14.4 ms with 3,
+// 15.1 with 4; 8 flies, 8 steps, where 3 leave latency uncovered: 122 us, 107 with 4).
+constexpr int kDeliverBlocks = 3;
 constexpr int kWindowEdges = 4;     // edges a lane of the delivery keeps in flight
 
 // Steps a window may hold (0: the run does not go by windows). It needs the raster to remember the
@@ -230,9 +234,12 @@ __device__ __forceinline__ float window_amount(const LifK& k, const Clk& clk, in
   return spike * r;
 }
 
+template <bool LISTED>
 struct WindowSmem {
-  static constexpr int CAP = kWindowBlock * kWindowBits;
+  static constexpr int CAP = kWindowBlock * kWindowSpikes;
   int wcnt[kWindowBlock / 32], wdeg[kWindowBlock / 32];
+  int wspk[LISTED ? 2 : 1][kWindowBlock / 32];   // spikes per warp of a task's words, alternate tasks
+  unsigned short item[LISTED ? CAP : 1];         // the round's spikes: (word of the task) * 32 + bit
   int pre[CAP];            // exclusive prefix of the spikers' out-degrees (all of them positive)
   int start[CAP];          // first outgoing edge
   long long to[CAP];       // ring offset of the fly in the write slot
@@ -248,42 +255,81 @@ __device__ __forceinline__ int spiker_of(const int* pre, int q, int lo, int hi) 
   return lo;
 }
 
-// Delivery of the window's spikes. A block takes kWindowBlock raster words at a time (or, `split`
-// > 0, that many 2^-split parts of words: few words then keep as many threads busy) and hands over their spikes in rounds of at most kWindowBits per thread; the round's edges are cut into
-// equal shares per warp, whatever the out-degrees (10^4 and beyond beside a mean of ~200). A warp
-// walks its share 32 positions at a time, one edge per lane: the spikers that start among the 32
-// positions are marked in a word, and a lane's spiker is the one before them plus the marks up to
-// its own position.
-template <bool FIXED>
-__device__ void window_deliver(const LifK& k, const Clk& clk, int s0, int K, int parts, WindowSmem& sm) {
-  constexpr int NW = kWindowBlock / 32;
+// Delivery of the window's spikes. A block takes kWindowBlock raster words at a time and hands over their
+// spikes in rounds of at most kWindowSpikes per thread. A persistent run of few items is bound by
+// latency and fires few cells per word: each thread takes the spikes of its own word. Per-step
+// launches list the block's spikes in item order first (LISTED) and share each round alike: where
+// many cells fire together a word holds up to 32 spikes, eight rounds of a few busy threads otherwise, and
+// the flies of a cell, whose targets share sectors, now go out together. 20 steps by windows of 6,
+// bursts under depression, us: 5,000 neurons, 16 flies 289 -> 117; by windows of 18: 20,000 neurons, 11
+// flies 170 -> 100; 70,000 neurons, 64 flies 2,240 -> 1,500. Sparse windows of one fly pay 0.5-1 us for
+// the list, which the persistent run's six windows of a 10 ms frame would feel (56 -> 63 us).
+// The round's edges are cut into `parts` shares, one per block that takes the same words (few words
+// then keep as many threads busy), and those into equal shares per warp, whatever the out-degrees
+// (10^4 and beyond beside a mean of ~200). A warp walks its share 32 positions at a time, one edge
+// per lane: the spikers that start among the 32 positions are marked in a word, and a lane's spiker
+// is the one before them plus the marks up to its own position.
+template <bool FIXED, bool LISTED>
+__device__ void window_deliver(const LifK& k, const Clk& clk, int s0, int K, int parts, WindowSmem<LISTED>& sm) {
+  constexpr int NW = kWindowBlock / 32, CAP = WindowSmem<LISTED>::CAP;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned upto = 0xffffffffu >> (31 - lane);            // this lane and those before it
   const size_t slot = (size_t)k.n * k.batch;
   const int w0 = k.t_begin >> 5, nw = ((k.t_end + 31) >> 5) - w0;
   const long long total = (long long)nw * K, tasks = (total + kWindowBlock - 1) / kWindowBlock * parts;
   unsigned long long events = 0;
-  for (long long task = blockIdx.x; task < tasks; task += gridDim.x) {
+  int flip = 0;
+  for (long long task = blockIdx.x; task < tasks; task += gridDim.x, flip ^= 1) {
     const int part = (int)(task % parts);
-    const unsigned u = (unsigned)(task / parts) * kWindowBlock + threadIdx.x;   // n * batch * K / 32 < 2^31
+    const unsigned u0 = (unsigned)(task / parts) * kWindowBlock, u = u0 + threadIdx.x;   // n * batch * K / 32 < 2^31
     const int j = (int)(u / (unsigned)nw), w = w0 + (int)(u - (unsigned)j * (unsigned)nw), s = s0 + j;
     unsigned bits = u < total ? k.raster[raster_row(k, clk, s) + w] : 0u;
     const size_t ws = (size_t)slot_after(clk.ring_pos, s + k.n_delay, k.R) * slot;
-    while (__syncthreads_or(bits != 0)) {                      // also: the shared lists are free again
-      int cnt = 0, sum = 0;
-      int e0[kWindowBits], deg[kWindowBits], fly[kWindowBits];
-      float x[kWindowBits];
+    int rank = 0, spikes = 0;                                  // of the word's first spike in the list, of all words
+    if (LISTED) {
+      const int mine_spk = __popc(bits), incl = warp_scan(mine_spk);
+      if (lane == 31) sm.wspk[flip][warp] = incl;
+      __syncthreads();
+      rank = incl - mine_spk;
 #pragma unroll
-      for (int q = 0; q < kWindowBits; ++q) {
+      for (int q = 0; q < NW; ++q) {
+        if (q < warp) rank += sm.wspk[flip][q];
+        spikes += sm.wspk[flip][q];
+      }
+    }
+    for (int r0 = 0; LISTED ? r0 < spikes : __syncthreads_or(bits != 0); r0 += CAP) {   // also: the shared arrays are free
+      const int m = spikes - r0 < CAP ? spikes - r0 : CAP, per = (m + kWindowBlock - 1) / kWindowBlock;
+      if (LISTED) {
+        for (; bits && rank < r0 + m; ++rank, bits &= bits - 1)
+          sm.item[rank - r0] = (unsigned short)(threadIdx.x * 32 + __ffs(bits) - 1);
+        __syncthreads();
+      }
+      int cnt = 0, sum = 0;
+      int e0[kWindowSpikes], deg[kWindowSpikes], fly[kWindowSpikes];
+      size_t at_step[kWindowSpikes];                                  // write slot (LISTED: a list mixes steps)
+      float x[kWindowSpikes];
+#pragma unroll
+      for (int q = 0; q < kWindowSpikes; ++q) {
         deg[q] = 0;
-        if (bits) {
-          const int bit = __ffs(bits) - 1, t = w * 32 + bit, i = neuron_of(k, t);
-          bits &= bits - 1;
+        if (LISTED ? q < per && (int)threadIdx.x * per + q < m : bits != 0) {
+          int bit, jq = j, wq = w;
+          if (LISTED) {
+            const int it = sm.item[threadIdx.x * per + q];
+            const unsigned uq = u0 + (it >> 5);
+            bit = it & 31;
+            jq = (int)(uq / (unsigned)nw);
+            wq = w0 + (int)(uq - (unsigned)jq * (unsigned)nw);
+            at_step[q] = (size_t)slot_after(clk.ring_pos, s0 + jq + k.n_delay, k.R) * slot;
+          } else {
+            bit = __ffs(bits) - 1;
+            bits &= bits - 1;
+          }
+          const int t = wq * 32 + bit, i = neuron_of(k, t);
           fly[q] = t - i * k.batch;
           e0[q] = __ldg(&k.out_ptr[i]);
           deg[q] = __ldg(&k.out_ptr[i + 1]) - e0[q];
           if (FIXED) {
-            x[q] = window_amount(k, clk, s0, s, (size_t)t, i, fly[q], w, bit);
+            x[q] = window_amount(k, clk, s0, s0 + jq, (size_t)t, i, fly[q], wq, bit);
             if (x[q] == 0.0f) deg[q] = 0;
           }
           cnt += deg[q] > 0;
@@ -301,11 +347,11 @@ __device__ void window_deliver(const LifK& k, const Clk& clk, int s0, int K, int
         E += sm.wdeg[q];
       }
 #pragma unroll
-      for (int q = 0; q < kWindowBits; ++q) {
+      for (int q = 0; q < kWindowSpikes; ++q) {
         if (deg[q] <= 0) continue;
         sm.pre[pos] = run;
         sm.start[pos] = e0[q];
-        sm.to[pos] = (long long)(ws + fly[q]);
+        sm.to[pos] = (long long)((LISTED ? at_step[q] : ws) + fly[q]);
         if (FIXED) sm.x[pos] = x[q];
         run += deg[q];
         ++pos;
@@ -365,9 +411,9 @@ __global__ void __launch_bounds__(kWindowBlock, FIXED ? 4 : 6) lif_window_update
 }
 
 template <bool FIXED>
-__global__ void __launch_bounds__(kWindowBlock) lif_window_deliver_kernel(LifK k, int s0, int K, int parts) {
-  __shared__ WindowSmem sm;
-  window_deliver<FIXED>(k, read_clock(k), s0, K, parts, sm);
+__global__ void __launch_bounds__(kWindowBlock, kDeliverBlocks) lif_window_deliver_kernel(LifK k, int s0, int K, int parts) {
+  __shared__ WindowSmem<true> sm;
+  window_deliver<FIXED, true>(k, read_clock(k), s0, K, parts, sm);
 }
 
 __global__ void __launch_bounds__(kWindowBlock) lif_window_finish_kernel(LifK k) {
@@ -377,7 +423,7 @@ __global__ void __launch_bounds__(kWindowBlock) lif_window_finish_kernel(LifK k)
 // Persistent launch: every window of the run in one cooperative kernel.
 template <bool FIXED, bool STD>
 __global__ void __launch_bounds__(kWindowBlock, FIXED ? 3 : 4) lif_window_persistent_kernel(LifK k, int kmax, int span, int parts) {
-  __shared__ WindowSmem sm;
+  __shared__ WindowSmem<false> sm;
   const Clk clk = read_clock(k);
   int generation = 0;
   for (int s0 = 0; s0 < k.nsteps; s0 += kmax) {
@@ -387,7 +433,7 @@ __global__ void __launch_bounds__(kWindowBlock, FIXED ? 3 : 4) lif_window_persis
       window_update<FIXED, STD, kAheadFew>(k, clk, s0, K, base, span);
     if (!grid_barrier(k.sync, k.status, generation, s0)) return;
     if (last && blockIdx.x == 0 && !(k.flags & FLYB_LIF_NO_ADVANCE)) advance_clock(k, clk);   // all have read it
-    window_deliver<FIXED>(k, clk, s0, K, parts, sm);
+    window_deliver<FIXED, false>(k, clk, s0, K, parts, sm);
     if (last && !STD) return;
     if (!grid_barrier(k.sync, k.status, generation, s0)) return;
   }
@@ -453,7 +499,7 @@ static int run_lif_windows(const LifK& k, int kmax, cudaStream_t st) {
         done += n;
       }
     } else if (!(k.flags & FLYB_LIF_PULL_DELIVERY)) {
-      lif_window_deliver_kernel<FIXED><<<sms * 4, kWindowBlock, 0, st>>>(k, s0, K, deliver_parts(k, K, sms * 4));
+      lif_window_deliver_kernel<FIXED><<<sms * kDeliverBlocks, kWindowBlock, 0, st>>>(k, s0, K, deliver_parts(k, K, sms * kDeliverBlocks));
       FLYB_CHECK_LAUNCH();
     }
     s0 += K;
