@@ -11,7 +11,7 @@
 // deterministic and equal to the C restatement in oracle/flyoracle.c bit for bit.
 //
 // Runs of more than one step go by delay windows (lif_window.cuh); the per-step kernels here run
-// single steps, neuron ranges, episode counters and runs without a raster.
+// single steps, neuron ranges, episode counters, runs without a raster and where window_steps leaves it to them.
 //
 // Layout: state [n][batch] (fly-minor), ring [R][n][batch]; work item t = i * batch + b.
 #include <type_traits>
@@ -1500,12 +1500,13 @@ template <int BLOCK, bool FIXED>
 static int run_lif(const LifK& k, int want, int launch, int grid_cap, int staged, cudaStream_t st) {
   int ipt = want ? want : 4;
   if (ipt != 1 && ipt != 2 && ipt != 4) return FLYB_EINVAL;
-  if (const int K = window_steps(k)) {
+  const bool stages = staged && launch == FLYB_LAUNCH_STEP && stageable(k);
+  if (const int K = window_steps(k, launch, stages, FIXED ? 8 : 4)) {
     if constexpr (FIXED)        // depression runs on the fixed ring only
       if (k.flags & FLYB_LIF_STD) return run_by_windows<FIXED, true>(k, K, launch, grid_cap, st);
     return run_by_windows<FIXED, false>(k, K, launch, grid_cap, st);
   }
-  if (staged && launch == FLYB_LAUNCH_STEP && stageable(k))
+  if (stages)
     return ipt == 4 ? run_lif_staged<BLOCK, FIXED, 4>(k, grid_cap, st) : run_lif_staged<BLOCK, FIXED, 2>(k, grid_cap, st);
   while (ipt > 1 && !vectorizable(k, ipt)) ipt >>= 1;
   if (ipt == 4) return run_lif_ipt<BLOCK, FIXED, 4>(k, launch, grid_cap, st);

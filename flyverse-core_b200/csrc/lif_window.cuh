@@ -37,13 +37,30 @@ constexpr int kDeliverBlocks = 3;
 constexpr int kWindowEdges = 4;     // edges a lane of the delivery keeps in flight
 
 // Steps a window may hold (0: the run does not go by windows). It needs the raster to remember the
-// window's spikes; episode counters gate single steps and stay with the per-step kernels.
-static int window_steps(const LifK& k) {
+// window's spikes; episode counters gate single steps and stay with the per-step kernels. Two rules
+// leave them per-step launches that scatter their spikes, where those are the faster:
+//  - launches that ask for the staged or the deferred kernel, where a ring slot is larger than a sixth
+//    of the L2: the K slots of a window at dense firing then go through DRAM, the one slot of a step
+//    less so (20 steps at a delay of 18, all cells bursting, deferred kernel against windows, ms:
+//    70,000 neurons, 256 flies, 72 MB 8.8 / 11.6; 40 flies on the fixed ring, 22 MB 2.0 / 2.4; but 64
+//    flies, 18 MB 2.9 / 1.9), or where the windows hold two steps only (20,000 neurons, 11 flies,
+//    staged, three steps at a delay of 2: 44 us, by windows 56);
+//  - depressing runs of two or three steps by windows of two, whose closing pass costs more than the
+//    windows save (20,000 neurons, 11 flies, two steps: 31 us, by windows 37).
+constexpr long long kWindowSlotBytes = 20ll << 20;
+
+static int window_steps(const LifK& k, int launch, bool staged, int ring_bytes) {
   if (!k.raster || k.nsteps < 2 || k.n_delay < 2 || (k.flags & FLYB_LIF_EPISODES)) return 0;
   int K = k.n_delay < k.nsteps ? k.n_delay : k.nsteps;
   if (k.raster_slots > 0 && K > k.raster_slots) K = k.raster_slots;
   if (K > kWindowMax) K = kWindowMax;
-  return K >= 2 ? K : 0;
+  if (K < 2) return 0;
+  if (launch == FLYB_LAUNCH_STEP && !(k.flags & FLYB_LIF_PULL_DELIVERY)) {
+    const long long slot_bytes = (long long)k.n * k.batch * ring_bytes;
+    if ((staged || k.spike_list) && (K == 2 || slot_bytes > kWindowSlotBytes)) return 0;
+    if ((k.flags & FLYB_LIF_STD) && K == 2 && k.nsteps < 4) return 0;
+  }
+  return K;
 }
 
 __device__ __forceinline__ size_t raster_row(const LifK& k, const Clk& clk, int s) {
