@@ -11,7 +11,7 @@
 // deterministic and equal to the C restatement in oracle/flyoracle.c bit for bit.
 //
 // Runs of more than one step go by delay windows (lif_window.cuh); the per-step kernels here run
-// single steps, neuron ranges, episode counters, runs without a raster and where window_steps leaves it to them.
+// single steps, episode counters, runs without a raster and where window_steps leaves it to them.
 //
 // Layout: state [n][batch] (fly-minor), ring [R][n][batch]; work item t = i * batch + b.
 #include <type_traits>

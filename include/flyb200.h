@@ -96,7 +96,8 @@ int launch_means(void** p, int n, int groups, int batch, int stride, void* strea
 #define FLYB_LAUNCH_PERSISTENT 1   /* one cooperative launch for all steps                    */
 /* An LIF run of nsteps >= 2 with a raster, n_delay >= 2 and no episode counters goes by delay
  * windows under both launch modes: up to min(n_delay, raster_slots, 32) steps per pass over the
- * state, then the delivery of their spikes (a pull: windows of at most two groups). block and items_per_thread shape single steps only. staged and
+ * state, then the delivery of their spikes (a pull: windows of at most two groups); runs over
+ * neuron ranges too. block and items_per_thread shape single steps only. staged and
  * FLYB_LIF_DEFER_DELIVERY keep their per-step kernels where a ring slot exceeds 20 MiB or a window
  * would hold two steps, else they shape single steps only.                                      */
 
