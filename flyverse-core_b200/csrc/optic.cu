@@ -293,20 +293,28 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
     }
     return 0;
   }
+  const long long need = optic_items<LPR>(k.m, k.n_long);
+  const bool single = k.nsteps == 1 && k.dr_valid;
+  if (single && grid_cap <= 0) {
+    // one substep on a carried dr has nothing to carry over a barrier: a block per item, dealt out by the
+    // hardware, needs no counts to be cleared first (3,000 units, two flies 22.6 -> 20 us a call;
+    // 20,000 units, 300 entries each, 256 flies 443 -> 341)
+    optic_step_kernel<W, NV, F, LPR, U, MINB><<<(unsigned)need, 256, 0, st>>>(k, 0);
+    return (int)cudaGetLastError();
+  }
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, optic_persistent_kernel<W, NV, F, LPR, U, MINB>, 256, 0);
   long long grid = (long long)sms * per_sm;
-  const long long need = optic_items<LPR>(k.m, k.n_long);
   if (grid > need) grid = need;
   if (grid_cap > 0 && grid > grid_cap) grid = grid_cap;
   if (grid < 1) return FLYB_ECOOP;
   cudaError_t e = cudaMemsetAsync(k.sync, 0, 2 * sizeof(int), st);   // barrier and item counts
   if (e != cudaSuccess) return (int)e;
-  if (k.nsteps == 1 && k.dr_valid) {
-    // one substep on a carried dr reaches no grid barrier: an ordinary launch of `grid` blocks
-    // looping over the items, which other kernels may share the SMs with
+  if (single) {
+    // ... and under a cap it reaches no grid barrier: an ordinary launch of `grid` blocks looping over
+    // the items, which other kernels may share the SMs with
     optic_persistent_kernel<W, NV, F, LPR, U, MINB><<<(unsigned)grid, 256, 0, st>>>(k);
     return (int)cudaGetLastError();
   }
