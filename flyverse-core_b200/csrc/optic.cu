@@ -347,16 +347,21 @@ static int run_optic(const OpticK& k, int launch, int grid_cap, cudaStream_t st)
 // as it can: the gathers then run at the L2's rate instead of the issue rate (89,390 units, 6 M
 // entries, one substep: 12 flies 162 us with 16 lanes of one fly, 55 us with 4 lanes of four; 24
 // flies 294 -> 80; 64 flies 254 -> 115 us and 128 flies 416 -> 254 us with the registers bounded for
-// six and four blocks per SM). Rows above 75,776 give a row of 4 or 8 fly lanes half a warp (12 flies,
-// 89,390 units 59 -> 50 us; 50,000 units 32.5 -> 34.3, so not below). Narrow rows leave lanes over for entries; a
+// six and four blocks per SM). In a lobe of many rows, a row of 4 fly lanes (and one of 8 whose flies are
+// no vectors) takes half a warp instead of a whole one. The line lies at 47,360 rows, where that is no slower
+// at 20 or 67 entries per row, by either launch (us per substep, whole / half warp, persistent launch,
+// 67 entries: 12 flies 30,000 rows 24.5 / 24.5, 40,000 29.4 / 28.8, 50,000 35.0 / 33.5, 89,390 59.4 / 49.4;
+// 6 flies 40,000 rows 27.6 / 28.6, 50,000 33.3 / 33.2, 89,390 57.4 / 47.7; 7 flies 30,000 23.4 / 24.8, 50,000
+// 35.7 / 30.4). Three flies on four lanes of one do so in any lobe but a small one (12,000 rows 12.2 /
+// 12.6, 20,000 16.5 / 15.1, 50,000 of 20 entries 23.9 / 16.7). Narrow rows leave lanes over for entries; a
 // lobe of few rows gives each row a whole warp (LPR 32), so that its rows still fill the SMs. The
 // other variants are what the autotuner tries beside it; one that the vector width rules out runs
 // as variant 0, an unknown one is an error.
 static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cudaStream_t st) {
   const void* const arrays[] = {k.v, k.adapt, k.buf0, k.buf1, k.pr, k.spk, k.v_hist, k.inp_hist};
   const int B = k.batch, w = vector_width(B, arrays);
-  const bool few = k.m <= 148 * 64;          // rows that a warp each would still hold on the SMs
-  const bool many = k.m > 148 * 512;         // rows enough to halve their lanes without idling any
+  const bool few = k.m <= 9472;              // rows that a warp each would still hold on the 148 SMs
+  const bool many = k.m > 47360;             // rows enough to halve their lanes without idling any
 #define FLYB_RUN(...) return run_optic<__VA_ARGS__>(k, launch, cap, st)
   if (B > 256) return FLYB_ETOOBIG;
   if (variant < 0 || variant > 5) return FLYB_EINVAL;
@@ -410,7 +415,7 @@ static int run_optic_shape(const OpticK& k, int variant, int launch, int cap, cu
     FLYB_RUN(2, 4, 32, 32, 2, 4);
   }
   if (B == 2) FLYB_RUN(1, 1, 2, 16, 8, 4);
-  if (B <= 4) { if (many) FLYB_RUN(1, 1, 4, 16, 8, 4); else FLYB_RUN(1, 1, 4, 32, 8, 4); }
+  if (B <= 4) { if (few) FLYB_RUN(1, 1, 4, 32, 8, 4); else FLYB_RUN(1, 1, 4, 16, 8, 4); }
   if (B <= 8) { if (many) FLYB_RUN(1, 1, 8, 16, 8, 4); else FLYB_RUN(1, 1, 8, 32, 8, 4); }
   if (B <= 16) FLYB_RUN(1, 1, 16, 32, 8, 4);
   if (B <= 32) FLYB_RUN(1, 1, 32, 32, 8, 4);
