@@ -1764,6 +1764,14 @@ FLYB_API int flyb_lif_run(const flyb_lif_args* a, void* stream) {
   }
 }
 
+FLYB_API int flyb_lif_window_steps(const flyb_lif_args* a) {
+  LifK k;
+  if (make_lif_k(a, k)) return -1;
+  if (k.clock_k || k.slow_classes) return 0;
+  return window_steps(k, a->launch, a->staged && a->launch == FLYB_LAUNCH_STEP && stageable(k),
+                      a->ring_mode == FLYB_RING_FIXED ? 8 : 4);
+}
+
 FLYB_API int flyb_ring_deposit(int n, int batch, int ring_mode, const int* out_ptr, const int* out_edge,
                                const float* x, void* ring_slot, void* stream) {
   if (n <= 0 || batch <= 0 || !out_ptr || !out_edge || !x || !ring_slot) return FLYB_EINVAL;

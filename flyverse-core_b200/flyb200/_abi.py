@@ -129,6 +129,7 @@ SIGNATURES = {
     "flyb_lif_advance": [ct.POINTER(LifArgs), _VP],
     "flyb_lif_pull": [ct.POINTER(LifArgs), _VP],
     "flyb_lif_spike_capacity": [ct.POINTER(LifArgs)],
+    "flyb_lif_window_steps": [ct.POINTER(LifArgs)],
     "flyb_ring_deposit": [_I, _I, _I, _VP, _VP, _VP, _VP, _VP],
     "flyb_optic_run": [ct.POINTER(OpticArgs), _VP],
     "flyb_optic_run_noalloc": [ct.POINTER(OpticArgs), _VP],

@@ -1,10 +1,10 @@
 """Launch-parameter autotuner for the native steps, cached per (graph, batch, activity bucket).
 
 The best launch shape depends on the graph, the batch and how many cells spike per step. Calls of
-many steps go by delay windows: one cooperative launch or two launches per window, the spikes
+many steps mostly go by delay windows: one cooperative launch or two launches per window, the spikes
 scattered or pulled. Engines that step by single launches stream the state from HBM every step:
 there the register and the bulk-copy kernels, block sizes and deliveries differ. `tune_lif` times
-each candidate (launch mode x block size x items per thread x spike delivery) for a few steps on a
+each distinct candidate (launch mode x block size x items per thread x spike delivery) for a few steps on a
 copy of the live state, restores the state, installs the fastest and caches it under the key;
 `tune_optic` does the same for the optic substep's launch mode and kernel shape.
 """
@@ -63,9 +63,13 @@ def _time(fn, reps: int) -> float:
 
 
 def _one_by_one(brain, steps: int) -> None:
-    """`steps` steps by single-step launches, as WholeFly takes them: the update by two ranges of neurons
-    (one over all of them would pull by itself), the clock, and under pull delivery a pull per
-    complete group."""
+    """`steps` steps by single-step launches. A plain brain takes them whole; one that is stepped beside
+    other work (`single_steps`) as WholeFly takes them: the update by two ranges of neurons (one over
+    all of them would pull by itself), the clock, and under pull delivery a pull per complete group."""
+    if not getattr(brain, "single_steps", False):
+        for _ in range(steps):
+            brain.step(1)
+        return
     head = brain.n * 15 // 16 // 32 * 32
     for _ in range(steps):
         for first, count in ((0, head), (head, brain.n - head)):
@@ -93,32 +97,59 @@ def _time_one_by_one(brain, steps: int) -> float:
     return _time(graph.replay, 1) / steps
 
 
+def _time_run(brain, steps: int) -> float:
+    """Milliseconds per step of a call of `steps` steps."""
+    brain.step(2)
+    return _time(lambda: brain.step(steps), 1) / steps
+
+
+def _route(brain, candidate: tuple, steps: int) -> tuple:
+    """What tells the kernels of a call of `steps` steps under the installed candidate from another's:
+    by delay windows the launch mode and whether spikes are pulled, else the whole candidate."""
+    launch, _, _, delivery = candidate
+    return (launch, "pull" in delivery) if brain.window_steps(steps) else candidate
+
+
 def tune_lif(brain, steps: int = 10, candidates=LIF_CANDIDATES) -> dict:
     """Install and return the fastest LIF launch choice for this brain; state is left unchanged.
     A brain with per-neuron clocks or the slow receptor tone has one launch shape (the extended
-    kernel): nothing to tune. Calls of several steps run by delay windows, whose update has one
-    shape too: there the candidates differ in the launch mode and the delivery. A brain that
-    is stepped one step per launch (`single_steps`, set by WholeFly) is timed that way."""
+    kernel): nothing to tune. Calls of several steps mostly run by delay windows, where candidates
+    that differ in the launch mode and the delivery alone are the same kernels: each such route is
+    timed once, and among the candidates of the fastest the one with the fastest single steps is
+    installed, since the brain's calls of one step run its shape. A brain that is stepped one step
+    per launch (`single_steps`, set by WholeFly) is timed that way only."""
     if getattr(brain, "_kvec", None) is not None or getattr(brain, "slow", None) is not None:
         return {"launch": "step", "block": 256, "items_per_thread": 1, "delivery": "extended", "ms_per_step": None}
-    key = ("lif", graph_key(brain), brain.B, activity_bucket(brain), bool(getattr(brain, "single_steps", False)))
+    single = bool(getattr(brain, "single_steps", False))
+    key = ("lif", graph_key(brain), brain.B, activity_bucket(brain), single)
     if key in CACHE:
         _apply(brain, CACHE[key])
         return CACHE[key]
     saved = brain.state_dict()
-    results = {}
     if not brain.can_pull():             # pull delivery: count ring and 32-fly groups only
         candidates = [c for c in candidates if "pull" not in c[3]]
-    for launch, block, ipt, delivery in candidates:
-        _apply(brain, {"launch": launch, "block": block, "items_per_thread": ipt, "delivery": delivery})
-        if getattr(brain, "single_steps", False):
-            ms = _time_one_by_one(brain, steps)
-        else:
-            brain.step(2)
-            ms = _time(lambda: brain.step(steps), 1) / steps
-        results[(launch, block, ipt, delivery)] = ms
+
+    def timed(candidate, fn) -> float:
+        _apply(brain, dict(zip(("launch", "block", "items_per_thread", "delivery"), candidate)))
+        ms = fn(brain, steps)
         brain.load_state_dict(saved)
-    best = min(results, key=results.get)
+        return ms
+
+    if single:
+        results = {c: timed(c, _time_one_by_one) for c in candidates}
+        best = min(results, key=results.get)
+    else:
+        runs, route_of = {}, {}
+        for c in candidates:
+            _apply(brain, dict(zip(("launch", "block", "items_per_thread", "delivery"), c)))
+            route_of[c] = _route(brain, c, steps)
+            if route_of[c] not in runs:
+                runs[route_of[c]] = timed(c, _time_run)
+        results = {c: runs[route_of[c]] for c in candidates}
+        fastest = min(runs, key=runs.get)
+        alike = [c for c in candidates if route_of[c] == fastest]
+        ones = {c: timed(c, _time_one_by_one) for c in alike} if len(alike) > 1 else {alike[0]: 0.0}
+        best = min(ones, key=ones.get)
     choice = {"launch": best[0], "block": best[1], "items_per_thread": best[2], "delivery": best[3],
               "ms_per_step": results[best],
               "all": {f"{k[0]}-{k[3]}/{k[1]}/{k[2]}": v for k, v in results.items()}}

@@ -565,6 +565,18 @@ class Brain:
         self.t += n_steps * self.p.dt
         self.step_count += n_steps
 
+    def window_steps(self, n_steps: int) -> int:
+        """Steps per delay window of `step(n_steps)`; 0 where it runs the per-step kernels."""
+        a = self._args
+        a.flags, a.nsteps, a.uniforms = self._flags(False), int(n_steps), None
+        self._set_delivery(a, 0, 0)
+        self._set_pull(a)
+        a.n_first, a.n_count = 0, 0
+        k = int(self._lib.flyb_lif_window_steps(ct.byref(a)))
+        if k < 0:
+            raise RuntimeError("flyb_lif_window_steps: bad arguments")
+        return k
+
     def step_range(self, n_first: int, n_count: int) -> None:
         """Update neurons [n_first, n_first + n_count) by one step on the current stream, leaving
         the device clock where it is (FLYB_LIF_NO_ADVANCE): the ranges of one step may run on

@@ -258,6 +258,10 @@ int flyb_lif_pull(const flyb_lif_args* a, void* stream);
  * pointers from the device, so call it at set-up, not during stream capture. -1 on bad input. */
 long long flyb_lif_spike_capacity(const flyb_lif_args* a);
 
+/* Steps per delay window of the run that flyb_lif_run would make of these arguments; 0: it goes by the
+ * per-step kernels, -1: bad input. Host work only. No counterpart in the reference. */
+int flyb_lif_window_steps(const flyb_lif_args* a);
+
 /* Advance `clock` by a->nsteps and lower `fly_steps` (FLYB_LIF_EPISODES) as the end of a
  * flyb_lif_run does: for runs split over neuron ranges with FLYB_LIF_NO_ADVANCE, after all of
  * them. One small launch on `stream`. No counterpart in the reference (it has one update per step). */
