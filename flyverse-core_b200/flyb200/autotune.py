@@ -16,8 +16,9 @@ import math
 import numpy as np
 import torch
 
+from .optic import long_row_entries
+
 CACHE: dict = {}
-OPTIC_VARIANTS = 6          # flyb_optic_args.variant values; a batch width has a subset of them
 # (launch, block, items per thread, delivery): "fused" delivers spikes inside the update kernel,
 # "staged" runs per-step launches through the bulk-copy kernel, "defer" lists the spikers and
 # delivers them from a second, load-balanced kernel, "staged-defer" does both
@@ -168,10 +169,29 @@ def _apply(brain, choice: dict) -> None:
     brain._make_args()
 
 
-# Row lengths above which a row is shared by a whole block (OpticCore.set_long_rows): the split
-# pays at many flies per row gather; at one fly a row of a few hundred entries is better left to
-# its warp slot.
-OPTIC_LONG_ROWS = (192, 384, 512, 768, 1024, 2048)
+# Row lengths above which a row is shared by a whole block (OpticCore.set_long_rows), tried beside the
+# lobe's own default: the split pays at many flies per row gather and in small lobes; at one fly a
+# row of a few hundred entries of a large lobe is better left to its warp slot.
+OPTIC_LONG_ROWS = (96, 192, 384, 512, 768, 1024, 2048)
+
+
+def optic_variants(batch: int, width: int) -> tuple:
+    """The flyb_optic_args.variant values that are kernels of their own at a batch whose flies lie in
+    vectors of `width` (4, 2 or 1); the others are refused or run as variant 0."""
+    if batch == 1:
+        return 0, 1, 2, 3, 4
+    if batch <= 32 or width == 1:
+        return (0,)
+    if batch <= 64:
+        return (0, 1, 2, 3, 4, 5) if width == 4 else (0, 4)
+    if width == 2:
+        return (0,)
+    return (0, 1, 3) if batch <= 128 else (0, 1, 3, 5)
+
+
+def _vector_width(core) -> int:
+    arrays = (core.v_s, core.adapt_s, *core._bufs, core.pr_in, core.spk_in)
+    return next(w for w in (4, 2, 1) if core.B % w == 0 and all(x.data_ptr() % (4 * w) == 0 for x in arrays))
 
 
 def tune_optic(core, steps: int = 10) -> dict:
@@ -188,15 +208,12 @@ def tune_optic(core, steps: int = 10) -> dict:
         return CACHE[key]
     v, a = core.v_s.clone(), core.adapt_s.clone()
     results = {}
-    for long_row in OPTIC_LONG_ROWS:
+    for long_row in sorted({*OPTIC_LONG_ROWS, long_row_entries(core.W.nnz, core.B)}):
         core.set_long_rows(long_row)
         for launch in ("step",) if single else ("step", "persistent"):
-            for variant in range(OPTIC_VARIANTS):
+            for variant in optic_variants(core.B, _vector_width(core)):
                 core.launch, core.variant = launch, variant
-                try:
-                    core.substeps(2)
-                except RuntimeError:                 # no such shape for this batch width
-                    continue
+                core.substeps(2)
                 results[(launch, variant, long_row)] = _time(lambda: core.substeps(steps, carry=True), 1) / steps
                 core.v_s.copy_(v)
                 core.adapt_s.copy_(a)

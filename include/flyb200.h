@@ -484,8 +484,10 @@ typedef struct flyb_trace_args {
 int flyb_trace_scene_floats(int n_sph, int n_box, int n_pln);
 int flyb_trace(const flyb_trace_args* a, void* stream);
 
-/* Device facts for grid sizing: SM count and co-resident blocks per SM for the persistent
- * kernels at `block` threads. kind: 0 LIF, 1 optic, 2 adjoint. */
+/* Device facts for grid sizing: SM count and co-resident blocks per SM of a persistent kernel. kind: 0 the
+ * per-step LIF kernel at `block` threads (runs without a raster or with episode counters, single steps;
+ * delay windows run 256 threads, 4 blocks per SM on the count ring and 3 on the fixed ring), 1 the optic
+ * substep and 2 the adjoint in the shape of one fly in a lobe of more than 9,472 units (256 threads). */
 int flyb_occupancy(int kind, int block, int* sm_count, int* blocks_per_sm);
 
 /* Failure-detection self test: one thread polls `flag` (device int, never set by anyone) through the
