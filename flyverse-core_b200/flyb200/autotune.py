@@ -63,7 +63,7 @@ def _time(fn, reps: int) -> float:
     return s.elapsed_time(e) / reps
 
 
-def _one_by_one(brain, steps: int) -> None:
+def one_by_one(brain, steps: int) -> None:
     """`steps` steps by single-step launches. A plain brain takes them whole; one that is stepped beside
     other work (`single_steps`) as WholeFly takes them: the update by two ranges of neurons (one over
     all of them would pull by itself), the clock, and under pull delivery a pull per complete group."""
@@ -83,16 +83,16 @@ def _one_by_one(brain, steps: int) -> None:
 
 
 def _time_one_by_one(brain, steps: int) -> float:
-    """Milliseconds per step of `_one_by_one`, replayed from a CUDA graph: the host's time per launch is
+    """Milliseconds per step of `one_by_one`, replayed from a CUDA graph: the host's time per launch is
     not what the candidates differ in. The graph holds whole delivery groups from a group's start
     on, as a caller's graph should: a pull across a group end walks the input tables twice."""
     L = brain.pull_group if brain._pull_active() else 1
     steps = -(-steps // L) * L
-    _one_by_one(brain, 2 + (-(brain.step_count + 2)) % L)
+    one_by_one(brain, 2 + (-(brain.step_count + 2)) % L)
     stream, graph = torch.cuda.Stream(brain.device), torch.cuda.CUDAGraph()
     stream.wait_stream(torch.cuda.current_stream(brain.device))
     with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
-        _one_by_one(brain, steps)
+        one_by_one(brain, steps)
     torch.cuda.current_stream(brain.device).wait_stream(stream)
     graph.replay()
     return _time(graph.replay, 1) / steps

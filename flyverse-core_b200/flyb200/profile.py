@@ -6,7 +6,7 @@
                               [--optic-launch step|persistent] [--optic-variant 0] [--optic-grid 0] [--optic-long-row 0]
                               [--no-overlap]
     python -m flyb200.profile --breakdown [--batch 64] [--steps 50]
-    (--per-call K: K whole-fly steps per call, `--steps` calls; --settle S: S steps first, from CUDA graphs)
+    (--per-call K: K whole-fly or LIF steps per call, `--steps` calls; --settle S: S steps first, from CUDA graphs)
 
 Builds flyb200.synthetic.whole_fly_config5 (167,106 neurons, 25.6 M edges), warms up, then runs
 `--steps` steps of the chosen part. Used for the launch list and the per-kernel captures whose
@@ -144,8 +144,8 @@ def main() -> None:
     ap.add_argument("--breakdown", action="store_true")
     ap.add_argument("--settle", type=int, default=0, help="steps replayed from CUDA graphs of 20 before the "
                                                            "profiled ones (3,000: the steady firing the bench times)")
-    ap.add_argument("--per-call", type=int, default=1, help="whole-fly steps per WholeFly.step call (the pull "
-                                                             "delivers whole groups of steps within a call)")
+    ap.add_argument("--per-call", type=int, default=1, help="steps per WholeFly.step or Brain.step call "
+                                                             "(the pull delivers whole groups of steps within a call)")
     ap.add_argument("--lif-block", type=int, default=256)
     ap.add_argument("--lif-ipt", type=int, default=0, help="LIF items per thread (0: automatic)")
     ap.add_argument("--lif-staged", action="store_true", help="LIF step through the bulk-copy kernel")
@@ -196,7 +196,7 @@ def main() -> None:
         if args.part == "whole":
             eng.step(args.per_call)
         elif args.part == "lif":
-            eng.lif.step(1)
+            eng.lif.step(args.per_call)
         else:
             eng.optic.substeps(1, carry=True)
     torch.cuda.synchronize()
