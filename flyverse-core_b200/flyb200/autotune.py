@@ -214,7 +214,9 @@ def tune_optic(core, steps: int = 10) -> dict:
             for variant in optic_variants(core.B, _vector_width(core)):
                 core.launch, core.variant = launch, variant
                 core.substeps(2)
-                results[(launch, variant, long_row)] = _time(lambda: core.substeps(steps, carry=True), 1) / steps
+                # five calls: shapes 1 % apart alone may be 10 % apart beside other work (256 flies: variants 0
+                # and 5 at 460 and 457 us per substep, the whole fly 1.176 and 1.062 ms)
+                results[(launch, variant, long_row)] = _time(lambda: core.substeps(steps, carry=True), 5) / steps
                 core.v_s.copy_(v)
                 core.adapt_s.copy_(a)
     best = min(results, key=results.get)

@@ -304,7 +304,9 @@ typedef struct flyb_optic_args {
   int n_long;            /* long rows at the front of `rows`                         */
   float* v_hist;         /* optional [nsteps][m][batch]: v before each substep       */
   float* inp_hist;       /* optional [nsteps][m][batch]: input of each substep       */
-  int* status; int* sync;
+  int* status; int* sync; /* persistent launches: as in flyb_lif_args; cleared by each launch that
+                            uses it, so launches that may overlap need words of their own. One
+                            substep under FLYB_OPTIC_DR_VALID without a grid cap uses none */
 } flyb_optic_args;
 
 int flyb_optic_run(const flyb_optic_args* a, void* stream);

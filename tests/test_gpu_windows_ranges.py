@@ -28,8 +28,8 @@ def run_range(b, first, count, steps):
                                                            (6, "step", False, 0.3, 25), (7, "persistent", False, 0.3, 25),
                                                            (64, "step", True, 0.0, 3), (128, "step", True, 0.0, 2)])
 def test_range_runs_equal_single_steps(batch, launch, pull, std_u, steps, first, count):
-    if pull and count == 1500:
-        pytest.skip("a launch over all neurons pulls by itself")
+    if pull and count == 1500:            # a launch over all neurons would pull by itself
+        count = 1408
     a, b = brain(batch, launch, pull, std_u), brain(batch, launch, pull, std_u)
     for x in (a, b):
         x.step(21)
