@@ -214,13 +214,14 @@ def to_group_end(eng, at_least: int = 2) -> int:
     return k
 
 
-def capture(eng, steps: int):
+def capture(eng, steps: int, take=None):
+    """A CUDA graph of `steps` steps (`take(eng, steps)`, default eng.step)."""
     s = torch.cuda.Stream()
     s.wait_stream(torch.cuda.current_stream())
     g = torch.cuda.CUDAGraph()
     with torch.cuda.stream(s):
         with torch.cuda.graph(g, stream=s):
-            eng.step(steps)
+            take(eng, steps) if take else eng.step(steps)
     torch.cuda.current_stream().wait_stream(s)
     return g
 
@@ -278,16 +279,19 @@ def time_graph(g, reps) -> float:
 
 def kernel_roofline(eng, reps=20) -> dict:
     """The LIF step and the optic substep timed alone with CUDA events (B=64), after one untimed
-    call of each. The LIF is timed as the whole fly launches it, over one delivery group
-    (Brain.pull_group single steps, each the update by two ranges of neurons, and one pull) started at
-    a group boundary, per step: the bytes of lif_bytes_per_step are what such a step moves."""
+    call of each. The LIF is timed as the whole fly launches it: a graph of one delivery group
+    (Brain.pull_group single steps, each the update by two ranges of neurons, and one pull) from a
+    group boundary on, per step; the bytes of lif_bytes_per_step are what such a step moves."""
     from flyb200.autotune import one_by_one
     L = eng.lif.pull_group if eng.lif._pull_active() else 1
     eng.lif.step(to_group_end(eng, 1))
     one_by_one(eng.lif, L)
     eng.optic.substeps(1, carry=True)
+    g = capture(eng.lif, L, one_by_one)
+    g.replay()
     torch.cuda.synchronize()
-    lif_ms = events_time(lambda: one_by_one(eng.lif, L), reps) / L
+    lif_ms = events_time(g.replay, reps) / L
+    del g
     opt_ms = events_time(lambda: eng.optic.substeps(1, carry=True), reps)
     lif_b, opt_b = eng.lif_bytes_per_step(group=L), eng.optic_bytes_per_step()
     return {"lif_ms": lif_ms, "optic_ms": opt_ms, "lif_bytes": lif_b, "optic_bytes": opt_b, "lif_group": L}
