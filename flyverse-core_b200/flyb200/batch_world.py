@@ -95,8 +95,7 @@ class BatchWorld(World):
         """Eye positions (B, 3) and orientations forward/left/up (B, 3 each) for the next eye
         traces, copied into the device buffers that `trace_eye` (and a graph that captured it)
         reads; the copy is complete on return, so a graph may read it from any stream."""
-        self._queue_pose(eye, forward, left, up)
-        torch.cuda.current_stream(self.device).synchronize()
+        self._queue_pose(eye, forward, left, up).synchronize()
         self._pose_stream = None
 
     def _capturing(self) -> bool:
@@ -105,9 +104,9 @@ class BatchWorld(World):
         with torch.cuda.device(self.device):
             return torch.cuda.is_current_stream_capturing()
 
-    def _queue_pose(self, eye, forward, left, up) -> None:
-        """The poses' copy queued on the current stream: one block, staged in pinned memory (the
-        allocator keeps it until the copy has run)."""
+    def _queue_pose(self, eye, forward, left, up) -> torch.cuda.Stream:
+        """The poses' copy queued on the current stream, which is returned: one block, staged in pinned
+        memory (the allocator keeps it until the copy has run)."""
         if self._eye is None:
             raise ValueError("set_eye() first")
         if self._capturing():
@@ -119,8 +118,9 @@ class BatchWorld(World):
             pose[:, 3 * q:3 * q + 3] = np.asarray(v, dtype=np.float64).reshape(self.B, 3)
         host[self.B * 72:].view(np.float32).reshape(self.B, 3)[:] = np.asarray(eye, dtype=np.float32).reshape(self.B, 3)
         self._pose_block.copy_(staged, non_blocking=True)
-        self._pose_stream = torch.cuda.current_stream(self.device)
-        self._pose_copied.record(self._pose_stream)
+        self._pose_stream = stream = torch.cuda.current_stream(self.device)
+        self._pose_copied.record(stream)
+        return stream
 
     @torch.no_grad()
     def trace_eye(self, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -136,7 +136,7 @@ class BatchWorld(World):
                 stream.wait_event(self._pose_copied)
         return self._trace_eye(out)
 
-    def _trace_eye(self, out: torch.Tensor | None) -> torch.Tensor:
+    def _trace_eye(self, out: torch.Tensor | None, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
         device = self._ready()
         eye_dirs, w, n_col = self._eye
         if out is None:
@@ -144,7 +144,7 @@ class BatchWorld(World):
         elif out.shape != (self.B, n_col, 4) or out.dtype != torch.float32 or not out.is_contiguous():
             raise ValueError(f"out must be a contiguous float32 ({self.B}, {n_col}, 4) tensor")
         launch_trace(self._scene, self._scene_shape, self.detail, out, origins=self._eye_pos, eye_dirs=eye_dirs,
-                     pose=self._pose, weights=w, shared_origin=True, rays=n_col * w.numel(), batch=self.B)
+                     pose=self._pose, weights=w, shared_origin=True, rays=n_col * w.numel(), batch=self.B, stream=stream)
         return out
 
     def column_radiance(self, eye, forward, left, up, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -153,10 +153,9 @@ class BatchWorld(World):
         fly's scene, weighted and summed over each column's samples in sample order
         (batch_sim.py:192-201). Writes into `out` when given (e.g. FlyBrain's held radiance)."""
         # the trace follows on the same stream: nothing waits for the copy (two synchronising copies a
-        # frame kept the host from queueing the next: 64 eyes 146 -> 77 us per frame, one 63 -> 39),
+        # frame kept the host from queueing the next: 64 eyes 146 -> 77 us per frame, one 63 -> 38),
         # unless a captured trace, which may be replayed on any stream, reads the same poses
         if self._pose_captured:
             self.set_pose(eye, forward, left, up)
-        else:
-            self._queue_pose(eye, forward, left, up)
-        return self._trace_eye(out)
+            return self._trace_eye(out)
+        return self._trace_eye(out, self._queue_pose(eye, forward, left, up))

@@ -123,8 +123,8 @@ def pack_scene(w) -> np.ndarray:
 def launch_trace(scene: torch.Tensor, shape: tuple, detail: float, out: torch.Tensor, *, origins: torch.Tensor,
                  dirs: torch.Tensor | None = None, eye_dirs: torch.Tensor | None = None,
                  pose: torch.Tensor | None = None, weights: torch.Tensor | None = None, shared_origin: bool = False,
-                 rays: int, batch: int) -> None:
-    """One flyb_trace launch on the current stream (arguments as in include/flyb200.h)."""
+                 rays: int, batch: int, stream: torch.cuda.Stream | None = None) -> None:
+    """One flyb_trace launch on `stream`, the current one by default (arguments as in include/flyb200.h)."""
     if rays == 0:
         return
     tensors = [t for t in (scene, origins, dirs, eye_dirs, pose, weights, out) if t is not None]
@@ -137,7 +137,7 @@ def launch_trace(scene: torch.Tensor, shape: tuple, detail: float, out: torch.Te
                        shared_origin=int(shared_origin), samples=1 if weights is None else weights.numel(),
                        detail=float(detail), scene=_abi.ptr(scene), origins=_abi.ptr(origins), dirs=_abi.ptr(dirs),
                        eye_dirs=_abi.ptr(eye_dirs), pose=_abi.ptr(pose), weights=_abi.ptr(weights), out=_abi.ptr(out))
-    stream = torch.cuda.current_stream(out.device).cuda_stream
+    stream = (torch.cuda.current_stream(out.device) if stream is None else stream).cuda_stream
     if torch.cuda.current_device() == out.device.index:
         rc = _abi.lib().flyb_trace(ct.byref(a), stream)
     else:
