@@ -91,7 +91,8 @@ def _time_one_by_one(brain, steps: int) -> float:
     one_by_one(brain, 2 + (-(brain.step_count + 2)) % L)
     stream, graph = torch.cuda.Stream(brain.device), torch.cuda.CUDAGraph()
     stream.wait_stream(torch.cuda.current_stream(brain.device))
-    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+    # (thread_local: other threads may allocate, copy and step their own brains meanwhile)
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
         one_by_one(brain, steps)
     torch.cuda.current_stream(brain.device).wait_stream(stream)
     graph.replay()
